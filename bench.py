@@ -626,7 +626,8 @@ def run_reference(args):
 # finest-level smoother kernel by the kind of plan the autotuner picked
 SMOOTHER_KERNEL = {
     "rowtile": "k_stag_rbx (finest-level row-tile fused red-black smooth of all three components)",
-    "tiled": "k_stag_rb (finest-level tiled fused red-black smooth)",
+    "tiled": "k_stag_zm (finest-level z-march, two red-black smooths of all three components), or k_stag_rb where the "
+             "march does not apply",
     "colour": "k_stag_gs (finest-level colour sweep)",
     "rules": "finest-level smoother of the fixed size rules",
 }

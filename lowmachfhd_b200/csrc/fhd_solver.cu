@@ -156,14 +156,7 @@ static int build_mg(fhd_ctx* ctx, Multigrid<T>& M) {
                 L.alpha[c] = L.own_alpha0[c];
             }
         }
-        // the levels the row-tile smoother can take (rbx_geom: FP32, 3D,
-        // visc_type 1, x extent 64 to 256)
-        if (!std::is_same<T, double>::value && dim == 3 && ctx->visc == 1 && L.g.n[0] >= 64 &&
-            L.g.n[0] <= RBX_MAXNX)
-            for (int c = 0; c < 3; c++) {
-                L.rbx_diag[c] = A.alloc<T>(nc);
-                if (!L.rbx_diag[c]) return FHD_ERR_OOM;
-            }
+        L.zm_ok = dim == 3 && stag_zm_pick<T>(L.g, 1, ctx->sms, L.zm[0]) && stag_zm_pick<T>(L.g, 2, ctx->sms, L.zm[1]);
     }
     const int ncl = nlevs_mg(ctx->g0, ctx->p.mg_minwidth);
     M.c.resize(ncl);
@@ -310,15 +303,6 @@ static int prepare_T(fhd_ctx* ctx) {
         if (rc) return rc;
         C.alpha_scale = T(1);
     }
-    for (StagLevel<T>& L : M.s) {
-        if (!L.rbx_diag[0]) continue;
-        const StagOp<T> A = L.op();
-        const int nb = flat_blocks(L.g.nc);
-        for (int c = 0; c < 3; c++) {
-            k_stag_diag1<T, 3><<<nb, 256, 0, st>>>(L.g.nc, L.rbx_diag[c], L.alpha[c], L.alpha_scale, L.beta, A.q);
-            FHD_POST(ctx);
-        }
-    }
     // pressure multigrid coefficients: alphainv on the finest level
     {
         const int nb = flat_blocks(nc0);
@@ -370,6 +354,22 @@ static int prepare_T(fhd_ctx* ctx) {
 template <typename T>
 static int tune_levels(fhd_ctx* ctx);
 
+// the diagonals of the levels whose plan (forced or imported) is the
+// row-tile smooth
+static int rbx_diagonals(fhd_ctx* ctx) {
+    for (StagLevel<float>& L : ctx->mg32.s) {
+        if (L.plan.kind != 2) continue;
+        const StagOp<float> A = L.op();
+        for (int c = 0; c < 3; c++) {
+            if (!L.rbx_diag[c] && !(L.rbx_diag[c] = ctx->arena.alloc<float>(L.g.nc))) return FHD_ERR_OOM;
+            k_stag_diag1<float, 3><<<flat_blocks(L.g.nc), 256, 0, ctx->stream>>>(L.g.nc, L.rbx_diag[c], L.alpha[c],
+                                                                               L.alpha_scale, L.beta, A.q);
+            FHD_POST(ctx);
+        }
+    }
+    return 0;
+}
+
 int prepare(fhd_ctx* ctx, const double* const alpha_fc[], const double* beta, const double* const beta_ed[],
             const double* gamma, double theta) {
     const int dim = ctx->dim;
@@ -380,7 +380,8 @@ int prepare(fhd_ctx* ctx, const double* const alpha_fc[], const double* beta, co
     ctx->theta = theta;
     if (ctx->prec == FHD_PREC_MIXED) {
         int rc = prepare_T<float>(ctx);
-        return rc ? rc : tune_levels<float>(ctx);
+        if (!rc) rc = tune_levels<float>(ctx);
+        return rc ? rc : rbx_diagonals(ctx);
     }
     int rc = prepare_T<double>(ctx);
     return rc ? rc : tune_levels<double>(ctx);
@@ -650,8 +651,80 @@ static int stag_smooths_planned(fhd_ctx* ctx, StagLevel<T>& L, const SmoothPlan&
     return 0;
 }
 
+// whether a level smooths with the z-march: 3D, even extents of at least
+// four cells, constant viscosity without cross terms; not where a caller
+// forced or imported a plan, or asked for colour launches (fhd_ctx_set_fused
+// 0).  It is the fastest form at every size it takes (a pair of smooths,
+// FP32, before and now: 40^3 52 -> 9 us, 128^3 64 -> 44, 192^3 238 -> 113,
+// 256^3 349 -> 280; FP64 128^3 136 -> 99), so no plan is timed against it.
 template <typename T>
-static int stag_smooths(fhd_ctx* ctx, StagLevel<T>& L, int count) {
+static bool zm_use(fhd_ctx* ctx, const StagLevel<T>& L) {
+    return L.zm_ok && ctx->visc == 1 && ctx->fused_mode != 0 && ctx->p.stag_mg_smoother != 0 && !ctx->has_walls &&
+           (L.plan.kind < 0 || L.plan.march) && stag_aligned(L, ctx->dim);
+}
+
+// one launch of ns smooths phi -> tmp of every component; the two buffers
+// then change names
+template <typename T>
+static int stag_zm_launch(fhd_ctx* ctx, StagLevel<T>& L, int ns, int zero) {
+    const ZMGeom& G = L.zm[ns - 1];
+    ZMArgs<T> R;
+    for (int c = 0; c < 3; c++) {
+        R.src[c] = L.phi[c];
+        R.dst[c] = L.tmp[c];
+        R.rhs[c] = L.rhs[c];
+    }
+    const bool timed = ctx->prof && L.g.nc == ctx->g0.nc;
+    if (timed) {
+        prof_mark(ctx, ctx->stream);
+        ctx->prof_bytes += rb_smooth_bytes(ctx, L);
+        ctx->prof_launches++;
+    }
+    const dim3 grd(G.tx * G.ty, G.chunks, 3);
+    const T omega = (T)ctx->p.stag_mg_omega;
+    if (ns == 1) {
+        if (int rc = rb_allow_smem(k_stag_zm<T, 1>, G.smem)) return rc;
+        k_stag_zm<T, 1><<<grd, G.threads, G.smem, ctx->stream>>>(L.g, G, L.op(), R, omega, zero);
+    } else {
+        if (int rc = rb_allow_smem(k_stag_zm<T, 2>, G.smem)) return rc;
+        k_stag_zm<T, 2><<<grd, G.threads, G.smem, ctx->stream>>>(L.g, G, L.op(), R, omega, zero);
+    }
+    if (int rc = post(ctx)) return rc;
+    if (timed) prof_mark(ctx, ctx->stream);
+    for (int c = 0; c < 3; c++) std::swap(L.phi[c], L.tmp[c]);
+    L.away = !L.away;
+    return 0;
+}
+
+// count smooths by the z-march, two per launch.  zero: the unknowns are zero
+// and need not be stored so.  home: the last smooths of the level in a
+// V-cycle, after which the unknowns lie where they lay at its start: when
+// the launches so far would leave them in the other buffer, the last pair
+// goes as two launches (or a lone last smooth is copied back).
+template <typename T>
+static int stag_zm_smooths(fhd_ctx* ctx, StagLevel<T>& L, int count, int zero, bool home) {
+    int pairs = count / 2, ones = count & 1;
+    const bool odd = home && (((pairs + ones) & 1) != 0) != L.away;
+    if (odd && pairs > 0) {
+        pairs--;
+        ones += 2;
+    }
+    for (; pairs > 0; pairs--, zero = 0)
+        if (int rc = stag_zm_launch(ctx, L, 2, zero)) return rc;
+    for (; ones > 0; ones--, zero = 0)
+        if (int rc = stag_zm_launch(ctx, L, 1, zero)) return rc;
+    if (home && L.away) {
+        for (int c = 0; c < 3; c++) {
+            FHD_CUDA_TRY(cudaMemcpyAsync(L.tmp[c], L.phi[c], sizeof(T) * L.g.nc, cudaMemcpyDeviceToDevice, ctx->stream));
+            std::swap(L.phi[c], L.tmp[c]);
+        }
+        L.away = false;
+    }
+    return 0;
+}
+
+template <typename T>
+static int stag_smooths(fhd_ctx* ctx, StagLevel<T>& L, int count, int zero = 0, bool home = true) {
     const int dim = ctx->dim;
     if (ctx->has_walls) {
         // the colours of the reference's smoother, each as Lphi and the
@@ -677,22 +750,10 @@ static int stag_smooths(fhd_ctx* ctx, StagLevel<T>& L, int count) {
     int m0 = 0;
     RBGeom G;
     const bool aligned = stag_aligned(L, dim);
-    if (L.plan.kind >= 0 && ctx->fused_mode != 0 && ctx->p.stag_mg_smoother != 0 && aligned && all_even(L.g))
+    if (zm_use(ctx, L)) return stag_zm_smooths(ctx, L, count, zero, home);
+    if (L.plan.kind >= 0 && !L.plan.march && ctx->fused_mode != 0 && ctx->p.stag_mg_smoother != 0 && aligned &&
+        all_even(L.g))
         return stag_smooths_planned(ctx, L, L.plan, count);
-    if constexpr (std::is_same<T, float>::value) {
-        RBXGeom X;
-        if (ctx->p.stag_mg_smoother != 0 && ctx->visc == 1 && count >= 2 && aligned && !rb_use(L.g) &&
-            ctx->fused_mode != 0 && rbx_geom(L.g, ctx->sms, (size_t)ctx->smem_optin, X)) {
-            float* a[3] = {L.phi[0], L.phi[1], L.phi[2]};
-            float* b[3] = {L.tmp[0], L.tmp[1], L.tmp[2]};
-            for (; m0 + 2 <= count; m0 += 2) {
-                int rc = stag_rbx_smooth(ctx, L, X, a, b);
-                if (rc) return rc;
-                rc = stag_rbx_smooth(ctx, L, X, b, a);
-                if (rc) return rc;
-            }
-        }
-    }
     if (ctx->p.stag_mg_smoother != 0 && count - m0 >= 2 && aligned && rb_use(L.g) &&
         rb_geom(L.g, 3, (int)sizeof(T), G)) {
         // pairs of fused smooths phi -> tmp -> phi
@@ -822,20 +883,31 @@ static int stag_coarse(fhd_ctx* ctx, Multigrid<T>& M, int lc) {
     return rc;
 }
 
+// zero0: the unknowns of level 0 start at zero, whatever is stored there
 template <typename T>
-static int stag_vcycle(fhd_ctx* ctx, Multigrid<T>& M) {
+static int stag_vcycle(fhd_ctx* ctx, Multigrid<T>& M, bool zero0) {
     const int nl = (int)M.s.size();
     const int dim = ctx->dim;
     cudaStream_t st = ctx->stream;
     // levels from lc down run in the coarse kernel, which zeroes their phi
     const int lc = stag_coarse_first(ctx, M);
     const int lt = lc < nl - 1 ? lc : nl - 1;  // last level of the per-level descent
-    for (int l = 1; l < lc; l++)
-        for (int c = 0; c < dim; c++) FHD_CUDA_TRY(cudaMemsetAsync(M.s[l].phi[c], 0, sizeof(T) * M.s[l].g.nc, st));
+    // a level that starts from zero by the z-march does not store the zeros
+    const int nd = ctx->p.stag_mg_nsmooths_down;
+    auto from_zero = [&](int l) {
+        const int n = l < nl - 1 ? nd : ctx->p.stag_mg_nsmooths_bottom;
+        return (l > 0 || zero0) && n > 0 && zm_use(ctx, M.s[l]);
+    };
+    for (int l = zero0 ? 0 : 1; l < lc; l++)
+        if (!from_zero(l))
+            for (int c = 0; c < dim; c++)
+                FHD_CUDA_TRY(cudaMemsetAsync(M.s[l].phi[c], 0, sizeof(T) * M.s[l].g.nc, st));
+    if (lc == 0 && zero0)  // the coarse kernel reads level 0's unknowns
+        for (int c = 0; c < dim; c++) FHD_CUDA_TRY(cudaMemsetAsync(M.s[0].phi[c], 0, sizeof(T) * M.s[0].g.nc, st));
     for (int l = 0; l < lt; l++) {
         StagLevel<T>& L = M.s[l];
         StagLevel<T>& C = M.s[l + 1];
-        int rc = stag_smooths(ctx, L, ctx->p.stag_mg_nsmooths_down);
+        int rc = stag_smooths(ctx, L, nd, from_zero(l), false);
         if (rc) return rc;
         rc = stag_residual(ctx, L);
         if (rc) return rc;
@@ -849,7 +921,8 @@ static int stag_vcycle(fhd_ctx* ctx, Multigrid<T>& M) {
         if (!rc) rc = zero_walls<T>(ctx, C.g, C.rhs[0], C.rhs[1], C.rhs[2]);
         if (rc) return rc;
     }
-    int rc = lc < nl ? stag_coarse(ctx, M, lc) : stag_smooths(ctx, M.s[nl - 1], ctx->p.stag_mg_nsmooths_bottom);
+    int rc = lc < nl ? stag_coarse(ctx, M, lc)
+                     : stag_smooths(ctx, M.s[nl - 1], ctx->p.stag_mg_nsmooths_bottom, from_zero(nl - 1));
     if (rc) return rc;
     for (int l = lt - 1; l >= 0; l--) {
         StagLevel<T>& L = M.s[l];
@@ -912,7 +985,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_maxabs(i64 n, const T* a, RedSl
 }
 
 template <typename T>
-static int stag_mg_run(fhd_ctx* ctx, Multigrid<T>& M);
+static int stag_mg_run(fhd_ctx* ctx, Multigrid<T>& M, bool zero0 = false);
 
 // one V-cycle of the multi-box hierarchy whose bottom, level lb, is the
 // fancy nested stag_mg_solver (stag_mg_solver.f90:447-555): levels lb ..
@@ -928,7 +1001,7 @@ static int stag_vcycle_fancy(fhd_ctx* ctx, Multigrid<T>& M, int lb) {
     for (int l = 0; l < lb; l++) {
         StagLevel<T>& L = M.s[l];
         StagLevel<T>& C = M.s[l + 1];
-        int rc = stag_smooths(ctx, L, ctx->p.stag_mg_nsmooths_down);
+        int rc = stag_smooths(ctx, L, ctx->p.stag_mg_nsmooths_down, 0, false);
         if (!rc) rc = stag_residual(ctx, L);
         if (rc) return rc;
         with_dim(dim, [&](auto D) {
@@ -964,12 +1037,17 @@ static int stag_vcycle_fancy(fhd_ctx* ctx, Multigrid<T>& M, int lb) {
 
 // stag_mg_solver (stag_mg_solver.f90:37-863) on level-0 phi/rhs of M
 template <typename T>
-static int stag_mg_run(fhd_ctx* ctx, Multigrid<T>& M) {
+static int stag_mg_cycles(fhd_ctx* ctx, Multigrid<T>& M, bool zero0) {
     const int dim = ctx->dim;
     const int maxv = ctx->p.stag_mg_max_vcycles;
     StagLevel<T>& L0 = M.s[0];
     const i64 nc = L0.g.nc;
-    if (int rc = zero_walls<T>(ctx, L0.g, L0.phi[0], L0.phi[1], L0.phi[2])) return rc;
+    if (zero0 && (maxv > 1 || maxv < 1)) {  // the zeros are read before the first smooth
+        for (int c = 0; c < dim; c++) FHD_CUDA_TRY(cudaMemsetAsync(L0.phi[c], 0, sizeof(T) * nc, ctx->stream));
+        zero0 = false;
+    }
+    if (!zero0)
+        if (int rc = zero_walls<T>(ctx, L0.g, L0.phi[0], L0.phi[1], L0.phi[2])) return rc;
     double resid0[3] = {0, 0, 0};
     if (maxv > 1) {
         int rc = stag_residual(ctx, L0);
@@ -998,7 +1076,7 @@ static int stag_mg_run(fhd_ctx* ctx, Multigrid<T>& M) {
     const bool nested = ctx->stag_fancy && maxv > 1 && M.s.size() == mg_of<T>(ctx).s.size() &&
                         ctx->stag_nl_box > 1 && ctx->stag_nl_box < (int)M.s.size();
     for (int vc = 1; vc <= maxv; vc++) {
-        int rc = nested ? stag_vcycle_fancy(ctx, M, ctx->stag_nl_box - 1) : stag_vcycle(ctx, M);
+        int rc = nested ? stag_vcycle_fancy(ctx, M, ctx->stag_nl_box - 1) : stag_vcycle(ctx, M, zero0 && vc == 1);
         if (rc) return rc;
         if (vc == maxv) break;
         rc = stag_residual(ctx, L0);
@@ -1015,6 +1093,19 @@ static int stag_mg_run(fhd_ctx* ctx, Multigrid<T>& M) {
     }
     ctx->vcycles += dim * maxv;
     return 0;
+}
+
+// stag_mg_solver; on an error the levels' buffers get their names back
+template <typename T>
+static int stag_mg_run(fhd_ctx* ctx, Multigrid<T>& M, bool zero0) {
+    const int rc = stag_mg_cycles(ctx, M, zero0);
+    if (rc)
+        for (auto& L : M.s)
+            if (L.away) {
+                for (int c = 0; c < 3; c++) std::swap(L.phi[c], L.tmp[c]);
+                L.away = false;
+            }
+    return rc;
 }
 
 // ---------------------------------------------------------------------
@@ -1119,7 +1210,7 @@ static std::map<std::string, int> g_tune_import;  // imported choices (candidate
 // the candidate lists (bumped whenever a list, its order or a candidate's
 // kernel changes), so a table from another GPU model or library version
 // selects nothing.
-constexpr int TUNE_CANDS_VERSION = 5;
+constexpr int TUNE_CANDS_VERSION = 6;
 
 static std::string tune_key_of(int dev, int which, int elem, int dim, int visc, const int n[3], int sms, int optin,
                                int smem_sm) {
@@ -1233,7 +1324,7 @@ static int tune_levels_locked(fhd_ctx* ctx, Multigrid<T>& M, std::vector<T*>& sc
     for (int l = 0; l < (int)M.s.size(); l++) {
         StagLevel<T>& L = M.s[l];
         L.plan = SmoothPlan();
-        if (l >= lcs || !all_even(L.g) || ctx->p.stag_mg_smoother == 0) continue;
+        if (l >= lcs || !all_even(L.g) || ctx->p.stag_mg_smoother == 0 || ctx->fused_mode == 0) continue;
         const std::string key = tune_key(ctx, L.g, 0, (int)sizeof(T));
         auto it = g_tune.find(key);
         if (force < 0 && it != g_tune.end()) {
@@ -1241,15 +1332,27 @@ static int tune_levels_locked(fhd_ctx* ctx, Multigrid<T>& M, std::vector<T*>& sc
             continue;
         }
         std::vector<SmoothPlan> cands = stag_cands(ctx, L);
+        const int nlist = (int)cands.size();
+        // the z-march: one past the list
+        SmoothPlan march;
+        march.kind = 1;
+        march.march = true;
+        march.ncand = nlist;
+        march.index = nlist;
+        const bool can_march = zm_use(ctx, L);
         if (force >= 0) {
-            L.plan = cands[(size_t)force < cands.size() ? force : 0];
-            L.plan.ncand = (int)cands.size();
+            if (force == nlist && can_march) {
+                L.plan = march;
+            } else {
+                L.plan = cands[force < nlist ? force : 0];
+                L.plan.ncand = nlist;
+            }
             continue;
         }
         auto im = g_tune_import.find(key);
-        if (im != g_tune_import.end() && im->second < (int)cands.size()) {
-            L.plan = cands[im->second];
-            L.plan.ncand = (int)cands.size();
+        if (im != g_tune_import.end() && (im->second < nlist || (im->second == nlist && can_march))) {
+            L.plan = im->second < nlist ? cands[im->second] : march;
+            L.plan.ncand = nlist;
             L.plan.index = im->second;
             g_tune[key] = L.plan;
             continue;
@@ -1262,9 +1365,18 @@ static int tune_levels_locked(fhd_ctx* ctx, Multigrid<T>& M, std::vector<T*>& sc
             S.rhs[c] = scratch[2 * dim + c];
         }
         if (!stag_aligned(S, dim)) continue;
+        if (can_march) {  // fastest wherever it runs (zm_use): timed for the record only
+            S.plan = march;
+            if (int rc = time_pairs(ctx, ev[0], ev[1], [&]() { return stag_zm_launch(ctx, S, 2, 0); }, march.us))
+                return rc;
+            L.plan = march;
+            g_tune[key] = L.plan;
+            continue;
+        }
         int best = -1;
         for (size_t i = 0; i < cands.size(); i++) {
             float us = 0.f;
+            if (cands[i].kind == 2) continue;  // (a level it takes marches)
             if (int rc = time_pairs(ctx, ev[0], ev[1], [&]() { return stag_smooths_planned(ctx, S, cands[i], 2); },
                                     us))
                 return rc;
@@ -1485,9 +1597,9 @@ static int precon_T(fhd_ctx* ctx, CSVec<double> b, SVec<double> x) {
     }
     StagLevel<T>& L0 = M.s[0];
     // velocity unknowns of the multigrid: the FP64 output itself, or FP32
-    // work arrays in the mixed preconditioner
+    // work arrays in the mixed preconditioner; the first multigrid solve
+    // starts from zero
     for (int c = 0; c < dim; c++) L0.phi[c] = fp64 ? (T*)x.c[c] : M.x_u[c];
-    for (int c = 0; c < dim; c++) FHD_CUDA_TRY(cudaMemsetAsync(L0.phi[c], 0, sizeof(T) * nc, st));
     auto set_rhs_from_b = [&]() -> int {
         for (int c = 0; c < dim; c++) {
             if (fp64) {
@@ -1586,7 +1698,7 @@ static int precon_T(fhd_ctx* ctx, CSVec<double> b, SVec<double> x) {
     int rc = 0;
     if (apt == 1) {
         if ((rc = set_rhs_from_b())) return rc;
-        if ((rc = stag_mg_run(ctx, M))) return rc;
+        if ((rc = stag_mg_run(ctx, M, true))) return rc;
         if ((rc = div_plus(b.c[dim]))) return rc;
         if ((rc = cc_solve(ctx, M))) return rc;
         with_dim(dim, [&](auto D) {
@@ -1603,7 +1715,7 @@ static int precon_T(fhd_ctx* ctx, CSVec<double> b, SVec<double> x) {
         if ((rc = bfbt ? visc_schur(fabs(theta) > 0.0, 0) : schur(kind, 1, 0))) return rc;
     } else if (apt == 2 || apt == 5) {
         if ((rc = set_rhs_from_b())) return rc;
-        if ((rc = stag_mg_run(ctx, M))) return rc;
+        if ((rc = stag_mg_run(ctx, M, true))) return rc;
         if ((rc = div_plus(b.c[dim]))) return rc;
         if (fabs(theta) > 0.0) {
             if ((rc = cc_solve(ctx, M))) return rc;
@@ -1613,7 +1725,7 @@ static int precon_T(fhd_ctx* ctx, CSVec<double> b, SVec<double> x) {
             return rc;
         if (apt == 5) {
             if ((rc = rhs_minus_grad_xp())) return rc;
-            if ((rc = stag_mg_run(ctx, M))) return rc;
+            if ((rc = stag_mg_run(ctx, M))) return rc;  // from the first solve's velocity
         }
         if ((rc = phi_to_x())) return rc;
     } else if (apt == 3) {
@@ -1624,11 +1736,11 @@ static int precon_T(fhd_ctx* ctx, CSVec<double> b, SVec<double> x) {
         }
         if ((rc = bfbt ? visc_schur(fabs(theta) > 0.0, 0) : schur(0, fabs(theta) > 0.0, 0))) return rc;
         if ((rc = rhs_minus_grad_xp())) return rc;
-        if ((rc = stag_mg_run(ctx, M))) return rc;
+        if ((rc = stag_mg_run(ctx, M, true))) return rc;
         if ((rc = phi_to_x())) return rc;
     } else {  // 4
         if ((rc = set_rhs_from_b())) return rc;
-        if ((rc = stag_mg_run(ctx, M))) return rc;
+        if ((rc = stag_mg_run(ctx, M, true))) return rc;
         const bool use_phi = fabs(theta) > 0.0;
         if (use_phi) {
             k_copy_conv<T, double><<<nb, 256, 0, st>>>(nc, M.c[0].rhs, b.c[dim], 1.0);
@@ -1692,7 +1804,7 @@ int stag_mg_solve_dev(fhd_ctx* ctx, double* const phi[], const double* const rhs
         int rc = stag_mg_run(ctx, M);
         if (rc) return rc;
         for (int c = 0; c < dim; c++) {
-            k_copy_conv<double, float><<<flat_blocks(nc), 256, 0, ctx->stream>>>(nc, phi[c], M.x_u[c], 1.0);
+            k_copy_conv<double, float><<<flat_blocks(nc), 256, 0, ctx->stream>>>(nc, phi[c], M.s[0].phi[c], 1.0);
             FHD_POST(ctx);
         }
         return 0;
@@ -2582,11 +2694,19 @@ int fhd_ctx_tune_info(fhd_ctx* c, int which, int level, int* kind, int* ncand, d
     if (ncand) *ncand = P->ncand;
     if (pair_us) *pair_us = P->us;
     if (shape) {
+        const ZMGeom* Z = P->march ? (c->prec == FHD_PREC_MIXED ? &c->mg32.s[level].zm[1] : &c->mg64.s[level].zm[1])
+                                   : nullptr;
         shape[0] = P->kind == 0 ? P->bx : P->kind == 1 ? P->rb.TX : P->kind == 2 ? c->n[0] : 0;
         shape[1] = P->kind == 0 ? P->by : P->kind == 1 ? P->rb.TY : P->kind == 2 ? P->rbx.TY : 0;
         shape[2] = P->kind == 1 ? P->rb.chunks : P->kind == 2 ? P->rbx.chunks : 0;
         shape[3] = P->kind == 2 ? P->rbx.per_sm : P->kind >= 0 ? 1 : 0;
         shape[4] = P->kind == 0 ? P->bx * P->by : P->kind == 1 ? P->rb.threads : P->kind == 2 ? P->rbx.threads : 0;
+        if (Z) {
+            shape[0] = 2 * Z->ip;
+            shape[1] = Z->TY;
+            shape[2] = Z->chunks;
+            shape[4] = Z->threads;
+        }
     }
     return FHD_OK;
 }

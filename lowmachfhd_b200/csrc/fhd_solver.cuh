@@ -12,6 +12,7 @@
 #include "fhd_vec.cuh"
 #include "fhd_rb.cuh"
 #include "fhd_walls.cuh"
+#include "fhd_zm.cuh"
 
 namespace fhd {
 
@@ -156,6 +157,7 @@ struct SmoothPlan {
     float us = 0.f;       // measured time of one smooth pair
     int ncand = 0;        // candidates the tuner considered
     int index = -1;       // position of this plan in the level's candidate list
+    bool march = false;   // kind 1 as the z-march of fhd_zm.cuh (one past the candidate list)
 };
 
 template <typename T>
@@ -175,8 +177,13 @@ struct StagLevel {
     T* rhs[3] = {nullptr, nullptr, nullptr};
     T* tmp[3] = {nullptr, nullptr, nullptr};   // residual / L phi
     T* diag[3] = {nullptr, nullptr, nullptr};  // two-pass smoother
+    // the z-march (fhd_zm.cuh) of one and of two smooths per launch, where
+    // the level's shape takes it
+    bool zm_ok = false;
+    ZMGeom zm[2];
+    bool away = false;  // phi and tmp are exchanged
     // the visc_type 1 diagonal alpha_scale alpha + 2 dim beta q, staged by the
-    // row-tile smoother in place of alpha (FP32 3D levels 64 to 256 wide)
+    // row-tile smoother in place of alpha (allocated when a plan takes it)
     T* rbx_diag[3] = {nullptr, nullptr, nullptr};
     StagOp<T> op() const {
         StagOp<T> A;
