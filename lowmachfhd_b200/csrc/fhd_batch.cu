@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(CS_THREADS) kb_cc_coarse(const CCCoarseArgs<T>
                                                           const Ctl* ctl, int mode) {
     const int b = order[blockIdx.x];
     if (!covers(ctl[b], mode)) return;
-    cc_coarse_run<T, 2>(args[b]);
+    cc_coarse_run<T, 2, true>(args[b]);
 }
 
 // ---------------------------------------------------------------------
@@ -1282,16 +1282,13 @@ int build(fhd_batch* B) {
         cq.n_bottom = B->p.mg_nsmooths_bottom;
         cq.phi = (T*)B->cphi[m0] + lc[(size_t)b * MAXL + m0].off;
         cq.rhs = (const T*)B->crhs[m0] + lc[(size_t)b * MAXL + m0].off;
-        off = 0;
         for (int q = 0; q < cq.nlev; q++) {
             const Grid& g = lc[(size_t)b * MAXL + m0 + q].g;
             cq.g[q] = g;
             for (int c = 0; c < 3; c++) cq.A[q].a[c] = (const T*)B->ones;
             cq.A[q].q = T(1.0 / (g.dx * g.dx));
-            cq.off[q] = (int)off;
-            off += (size_t)3 * (size_t)g.nc;
         }
-        B->smem_c = std::max(B->smem_c, off * sizeof(T));
+        B->smem_c = std::max(B->smem_c, cc_coarse_layout(cq, 2, true, budget));
     }
     B->sargs = dalloc<StagCoarseArgs<T>>(B, nb);
     B->cargs = dalloc<CCCoarseArgs<T>>(B, nb);

@@ -1483,15 +1483,11 @@ static int cc_coarse(fhd_ctx* ctx, Multigrid<T>& M, int lc) {
     a.n_bottom = ctx->p.mg_nsmooths_bottom;
     a.phi = M.c[lc].phi;
     a.rhs = M.c[lc].rhs;
-    size_t off = 0;
     for (int m = 0; m < a.nlev; m++) {
-        const CCLevel<T>& C = M.c[lc + m];
-        a.g[m] = C.g;
-        a.A[m] = C.op();
-        a.off[m] = (int)off;
-        off += (size_t)3 * (size_t)C.g.nc;
+        a.g[m] = M.c[lc + m].g;
+        a.A[m] = M.c[lc + m].op();
     }
-    const size_t smem = off * sizeof(T);
+    const size_t smem = cc_coarse_layout(a, ctx->dim, false, (size_t)ctx->smem_optin);
     int rc = 0;
     with_dim(ctx->dim, [&](auto D) {
         constexpr int DIM = decltype(D)::value;

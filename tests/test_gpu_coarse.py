@@ -55,6 +55,33 @@ def test_coarse_kernel_bitwise_fp64(cuda, dim, n, visc, kw):
     assert n1 < n0
 
 
+# edges of the coarse kernels: odd bottoms of uneven extents, rows longer than
+# the block, a single odd level, levels whose pressure coefficients do not fit
+# beside the unknowns (80^2, 24 x 16 x 20 in FP64), the Jacobi smoother
+EDGES = [
+    (3, [40, 24, 20], 1, {}),
+    (3, [10, 14, 6], 1, {}),
+    (3, [24, 16, 20], 1, {}),
+    (3, [5, 7, 3], 1, {}),
+    (2, [80, 80], 1, {}),
+    (2, [72, 56], 1, {}),
+    (2, [1100, 4], 1, {}),
+    (2, [4, 300], 1, {}),
+    (2, [35, 21], -1, {}),
+    (3, [16, 8, 4], 1, dict(stag_mg_smoother=0, stag_mg_omega=0.6)),
+    (3, [8, 8, 8], -1, dict(stag_mg_nsmooths_down=3, stag_mg_nsmooths_bottom=1, mg_nsmooths_up=1)),
+]
+
+
+@pytest.mark.parametrize("dim,n,visc,kw", EDGES)
+def test_coarse_kernel_edges(cuda, dim, n, visc, kw):
+    phi1, x1, n1 = _run(cuda, dim, n, visc, kw, 1)
+    phi0, x0, n0 = _run(cuda, dim, n, visc, kw, 0)
+    for a, b in zip(phi1 + x1, phi0 + x0):
+        assert np.array_equal(a, b)
+    assert n1 < n0
+
+
 @pytest.mark.parametrize("dim,n,visc", [(3, [32, 32, 32], 1), (3, [64, 64, 64], -1), (2, [128, 128], 2)])
 def test_coarse_kernel_mixed(cuda, dim, n, visc):
     phi1, x1, _ = _run(cuda, dim, n, visc, {}, 1, precision="mixed")
