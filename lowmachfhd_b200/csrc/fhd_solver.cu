@@ -1816,7 +1816,7 @@ int stag_mg_solve_dev(fhd_ctx* ctx, double* const phi[], const double* const rhs
 // ---------------------------------------------------------------------
 // apply_matrix (apply_matrix.f90:24-157), FP64 always
 // ---------------------------------------------------------------------
-int stokes_apply(fhd_ctx* ctx, CSVec<double> x, CSVec<double> rhs, SVec<double> out, int mode) {
+int stokes_apply(fhd_ctx* ctx, CSVec<double> x, CSVec<double> rhs, SVec<double> out, int mode, const double* inv) {
     StagOp<double> A;
     for (int c = 0; c < 3; c++) {
         A.alpha[c] = ctx->alpha_fc[c];
@@ -1831,7 +1831,7 @@ int stokes_apply(fhd_ctx* ctx, CSVec<double> x, CSVec<double> rhs, SVec<double> 
         with_dim_wall_visc(ctx->dim, ctx->visc, [&](auto D, auto V) {
             constexpr int DIM = decltype(D)::value, VISC = decltype(V)::value;
             k_stokes_apply_w<DIM, VISC><<<cell_grid(ctx->g0), cell_block(), 0, ctx->stream>>>(
-                ctx->g0, ctx->walls, A, x, rhs, out, mode, 1.0 / ctx->dx);
+                ctx->g0, ctx->walls, A, x, rhs, out, mode, 1.0 / ctx->dx, inv);
             rc |= post(ctx);
         });
         return rc;
@@ -1840,16 +1840,16 @@ int stokes_apply(fhd_ctx* ctx, CSVec<double> x, CSVec<double> rhs, SVec<double> 
         const double t1 = 1.0 / (12.0 * ctx->dx), t2 = 1.0 / (12.0 * ctx->dx * ctx->dx);
         if (ctx->dim == 2)
             k_stokes_apply4<2><<<cell_grid(ctx->g0), cell_block(), 0, ctx->stream>>>(ctx->g0, A, x, rhs, out, mode,
-                                                                                   1.0 / ctx->dx, t1, t2);
+                                                                                   1.0 / ctx->dx, t1, t2, inv);
         else
             k_stokes_apply4<3><<<cell_grid(ctx->g0), cell_block(), 0, ctx->stream>>>(ctx->g0, A, x, rhs, out, mode,
-                                                                                   1.0 / ctx->dx, t1, t2);
+                                                                                   1.0 / ctx->dx, t1, t2, inv);
         return post(ctx);
     }
     with_dim_visc(ctx->dim, ctx->visc, [&](auto D, auto V) {
         constexpr int DIM = decltype(D)::value, VISC = decltype(V)::value;
         k_stokes_apply<DIM, VISC><<<cell_grid(ctx->g0), cell_block(), 0, ctx->stream>>>(ctx->g0, A, x, rhs, out, mode,
-                                                                                      1.0 / ctx->dx);
+                                                                                      1.0 / ctx->dx, inv);
         rc |= post(ctx);
     });
     return rc;
@@ -2041,12 +2041,53 @@ static CSVec<double> csv(SVec<double> v) {
     return o;
 }
 
-static int wnorm2(fhd_ctx* ctx, CSVec<double> a, int slotid) {
+static int gs_blocks(i64 nc) {
+    const int b = flat_blocks(nc);
+    return b < GS_BLOCKS ? b : GS_BLOCKS;
+}
+
+// |a|^2 into a scalar slot, and its inverse root where asked
+static int wnorm2(fhd_ctx* ctx, CSVec<double> a, int slotid, double* inv = nullptr) {
     const i64 nc = ctx->g0.nc;
     const double wp = ctx->p.p_norm_weight;
-    k_sdot<double, double><<<flat_blocks(nc), RED_THREADS, 0, ctx->stream>>>(nc, ctx->dim + 1, a, a, wp * wp,
-                                                                          slot(ctx, slotid));
+    with_dim(ctx->dim, [&](auto D) {
+        k_norm2<decltype(D)::value + 1><<<gs_blocks(nc), RED_THREADS, 0, ctx->stream>>>(
+            nc, a, wp * wp, ctx->dscal + slotid, inv, ctx->gs.partials, ctx->gs.counter);
+    });
     return post(ctx);
+}
+
+// f(NV) with NV = nv as a constant, 1 <= nv <= GS_MAXV
+template <int N = GS_MAXV, class F>
+static void with_nv(int nv, F&& f) {
+    if constexpr (N > 1) {
+        if (nv < N) return with_nv<N - 1>(nv, f);
+    }
+    f(std::integral_constant<int, N>());
+}
+
+// the new Krylov vector w orthogonalised against u_0 .. u_{i-1}, as u_i
+static int orthogonalise(fhd_ctx* ctx, CSVec<double> w, SVec<double> ui, int i) {
+    const i64 nc = ctx->g0.nc, vstride = (i64)(ctx->dim + 1) * nc;
+    const double wp2 = ctx->p.p_norm_weight * ctx->p.p_norm_weight;
+    const int nb = gs_blocks(nc);
+    for (int pass = 0; pass < 2; pass++)
+        for (int k0 = 0; k0 < i; k0 += GS_MAXV) {
+            const int nv = i - k0 < GS_MAXV ? i - k0 : GS_MAXV;
+            with_dim(ctx->dim, [&](auto D) {
+                with_nv(nv, [&](auto N) {
+                    constexpr int NC = decltype(D)::value + 1, NV = decltype(N)::value;
+                    if (pass == 0)
+                        k_gs_dots<NC, NV><<<nb, RED_THREADS, 0, ctx->stream>>>(nc, w, ctx->V, vstride, k0, i, wp2,
+                                                                              ctx->gs);
+                    else
+                        k_gs_update<NC, NV><<<nb, RED_THREADS, 0, ctx->stream>>>(
+                            nc, k0 ? csv(ui) : w, ui, ctx->V, vstride, k0, i, k0 + nv == i, wp2, ctx->gs);
+                });
+            });
+            FHD_POST(ctx);
+        }
+    return 0;
 }
 
 int gmres_dev(fhd_ctx* ctx, CSVec<double> b, SVec<double> x, double* norm_pre_rhs, fhd_solve_stats* stout) {
@@ -2058,8 +2099,11 @@ int gmres_dev(fhd_ctx* ctx, CSVec<double> b, SVec<double> x, double* norm_pre_rh
     cudaStream_t st = ctx->stream;
     const int nb = flat_blocks(nc);
     const i64 vstride = (i64)ncomp * nc;
-    SVec<double> tmp = svec(ctx->tmp, dim, nc), r = svec(ctx->r, dim, nc), w = svec(ctx->w, dim, nc);
-    auto V = [&](int k) { return svec(ctx->V + (i64)k * vstride, dim, nc); };  // 0-based
+    SVec<double> tmp = svec(ctx->tmp, dim, nc), w = svec(ctx->w, dim, nc);
+    // Krylov vectors, 0-based, not scaled (fhd_vec.cuh); the first is the
+    // preconditioned residual itself
+    auto V = [&](int k) { return svec(ctx->V + (i64)k * vstride, dim, nc); };
+    const SVec<double> r = V(0);
     fhd_solve_stats S;
     memset(&S, 0, sizeof(S));
     ctx->vcycles = 0;
@@ -2080,19 +2124,19 @@ int gmres_dev(fhd_ctx* ctx, CSVec<double> b, SVec<double> x, double* norm_pre_rh
         if (stout) *stout = S;
         return 0;
     }
-    std::vector<double> H((m + 2) * (m + 2), 0.0), cs(m + 2), sn(m + 2), s(m + 2), y(m + 2);
+    std::vector<double> H((m + 2) * (m + 2), 0.0), cs(m + 2), sn(m + 2), s(m + 2), y(m + 2), len(m + 2);
     auto Hh = [&](int i, int j) -> double& { return H[i * (m + 2) + j]; };
     int total_iter = 0, iter = 0, i_copy = 0;
     double norm_resid = 0, norm_init_resid = 0, norm_resid_Stokes = 0, norm_init_Stokes = 0, norm_resid_est = 0;
     for (;;) {
         // tmp = b - A x
         if ((rc = stokes_apply(ctx, csv(x), b, tmp, 1))) return rc;
-        if ((rc = wnorm2(ctx, csv(tmp), S_NRM))) return rc;
+        if ((rc = wnorm2(ctx, csv(tmp), S_N2 + 1))) return rc;
         if ((rc = precon_graphed(ctx, csv(tmp), r))) return rc;
-        if ((rc = wnorm2(ctx, csv(r), S_NRM + 1))) return rc;
-        if ((rc = sync_scalars(ctx, S_NRM, 2))) return rc;
-        norm_resid_Stokes = sqrt(ctx->hscal[S_NRM]);
-        norm_resid = sqrt(ctx->hscal[S_NRM + 1]);
+        if ((rc = wnorm2(ctx, csv(r), S_N2, ctx->gs.inv))) return rc;
+        if ((rc = sync_scalars(ctx, S_N2, 2))) return rc;
+        norm_resid_Stokes = sqrt(ctx->hscal[S_N2 + 1]);
+        norm_resid = sqrt(ctx->hscal[S_N2]);
         if (iter == 0) {
             norm_init_Stokes = norm_resid_Stokes;
             norm_init_resid = norm_resid;
@@ -2115,43 +2159,23 @@ int gmres_dev(fhd_ctx* ctx, CSVec<double> b, SVec<double> x, double* norm_pre_rh
             break;
         }
         iter++;
-        k_scale_div<<<nb, 256, 0, st>>>(nc, ncomp, V(0), csv(r), norm_resid);
-        FHD_POST(ctx);
         std::fill(s.begin(), s.end(), 0.0);
-        s[1] = norm_resid;
+        s[1] = len[0] = norm_resid;
         for (int i = 1; i <= m; i++) {
             total_iter++;
             i_copy = i;
-            // the iteration's launches -- A v_{i-1}, the preconditioner,
-            // modified Gram-Schmidt with device-resident coefficients, the
-            // normalisation -- and the copy of the new Hessenberg column to
-            // the host: in graph mode 2 replayed as one graph per i, else
-            // launched one by one around the preconditioner's graph
+            // the iteration's launches -- A v_{i-1}, the preconditioner, the
+            // orthogonalisation with device-resident coefficients -- and the
+            // copy of the new Hessenberg column to the host: in graph mode 2
+            // replayed as one graph per i, else launched one by one around
+            // the preconditioner's graph
             const bool igraph = ctx->graph_mode == 2;
             auto body = [&]() -> int {
                 int r2;
-                if ((r2 = stokes_apply(ctx, csv(V(i - 1)), csv(V(i - 1)), tmp, 0))) return r2;
+                if ((r2 = stokes_apply(ctx, csv(V(i - 1)), csv(V(i - 1)), tmp, 0, ctx->gs.inv + i - 1))) return r2;
                 if ((r2 = igraph ? precon(ctx, csv(tmp), w) : precon_graphed(ctx, csv(tmp), w))) return r2;
-                for (int k = 1; k <= i; k++) {
-                    CSVec<double> none;
-                    for (int c = 0; c < 4; c++) none.c[c] = nullptr;
-                    k_mgs<<<nb, RED_THREADS, 0, st>>>(nc, ncomp, w, k > 1 ? csv(V(k - 2)) : none,
-                                                      k > 1 ? ctx->dscal + S_H + k - 1 : nullptr, csv(V(k - 1)),
-                                                      wp * wp, slot(ctx, S_H + k));
-                    FHD_POST(ctx);
-                }
-                {
-                    CSVec<double> none;
-                    for (int c = 0; c < 4; c++) none.c[c] = nullptr;
-                    k_mgs<<<nb, RED_THREADS, 0, st>>>(nc, ncomp, w, csv(V(i - 1)), ctx->dscal + S_H + i, none,
-                                                      wp * wp, slot(ctx, S_NRM));
-                    FHD_POST(ctx);
-                }
-                k_scale_by_norm<<<nb, 256, 0, st>>>(nc, ncomp, V(i), csv(w), ctx->dscal + S_NRM);
-                FHD_POST(ctx);
-                FHD_CUDA_TRY(cudaMemcpyAsync(ctx->hscal + S_H + 1, ctx->dscal + S_H + 1, sizeof(double) * i,
-                                             cudaMemcpyDeviceToHost, st));
-                FHD_CUDA_TRY(cudaMemcpyAsync(ctx->hscal + S_NRM, ctx->dscal + S_NRM, sizeof(double),
+                if ((r2 = orthogonalise(ctx, csv(w), V(i), i))) return r2;
+                FHD_CUDA_TRY(cudaMemcpyAsync(ctx->hscal + S_H, ctx->dscal + S_H, sizeof(double) * (S_N2 + i + 1),
                                              cudaMemcpyDeviceToHost, st));
                 return 0;
             };
@@ -2160,7 +2184,7 @@ int gmres_dev(fhd_ctx* ctx, CSVec<double> b, SVec<double> x, double* norm_pre_rh
             if ((rc = igraph ? graphed(ctx, ikey, body) : body())) return rc;
             FHD_CUDA_TRY(cudaStreamSynchronize(st));
             for (int k = 1; k <= i; k++) Hh(k, i) = ctx->hscal[S_H + k];
-            Hh(i + 1, i) = sqrt(ctx->hscal[S_NRM]);
+            Hh(i + 1, i) = len[i] = sqrt(ctx->hscal[S_N2 + i]);
             if (Hh(i + 1, i) == 0.0) {
                 set_last_error("gmres: error in orthogonalization");
                 return FHD_ERR_ORTHO_BREAKDOWN;
@@ -2208,7 +2232,7 @@ int gmres_dev(fhd_ctx* ctx, CSVec<double> b, SVec<double> x, double* norm_pre_rh
                 for (int jj = ii + 1; jj <= k + 1; jj++) acc += Hh(ii, jj) * y[jj];
                 y[ii] = (s[ii] - acc) / Hh(ii, ii);
             }
-            for (int it = 1; it <= i_copy; it++) ctx->hscal[S_Y + it - 1] = y[it];
+            for (int it = 1; it <= i_copy; it++) ctx->hscal[S_Y + it - 1] = y[it] / len[it - 1];
             FHD_CUDA_TRY(cudaMemcpyAsync(ctx->dscal + S_Y, ctx->hscal + S_Y, sizeof(double) * i_copy,
                                          cudaMemcpyHostToDevice, st));
             k_update_sol<<<nb, 256, 0, st>>>(nc, ncomp, x, ctx->V, vstride, ctx->dscal + S_Y, i_copy);
@@ -2417,17 +2441,20 @@ static int ctx_create(int dim, const int n_cells[3], const int max_grid_size[3],
     const i64 sv = (i64)(dim + 1) * nc;
     if (!rc) {
         c->V = c->arena.alloc<double>(sv * (c->m + 1));
-        c->r = c->arena.alloc<double>(sv);
         c->w = c->arena.alloc<double>(sv);
         c->tmp = c->arena.alloc<double>(sv);
         c->xs = c->arena.alloc<double>(sv);
         c->red_partials = c->arena.alloc<double>(RED_MAX_BLOCKS);
+        double* gs = c->arena.alloc<double>(4 * GS_MAXM + GS_MAXM * GS_MAXM + 2 * GS_MAXV * GS_BLOCKS);
         c->red_counter = (unsigned*)c->arena.alloc<double>(1);
         c->dscal = c->arena.alloc<double>(NSCAL);
         c->dev_err = (unsigned*)c->arena.alloc<double>(1);
-        if (!c->V || !c->r || !c->w || !c->tmp || !c->xs || !c->red_partials || !c->red_counter || !c->dscal ||
+        if (!c->V || !gs || !c->w || !c->tmp || !c->xs || !c->red_partials || !c->red_counter || !c->dscal ||
             !c->dev_err)
             rc = FHD_ERR_OOM;
+        else
+            c->gs = {c->dscal + S_H, c->dscal + S_N2,   gs, gs + GS_MAXM, gs + 2 * GS_MAXM, gs + 3 * GS_MAXM,
+                     gs + 4 * GS_MAXM, gs + 4 * GS_MAXM + GS_MAXM * GS_MAXM, c->red_counter};
     }
     if (!rc && !(c->hscal = pinned_scalars_acquire())) rc = FHD_ERR_OOM;
     if (!rc && cudaMemsetAsync(c->red_counter, 0, sizeof(double), c->stream) != cudaSuccess) rc = FHD_ERR_CUDA;

@@ -267,13 +267,13 @@ struct fhd_ctx {
     double theta = 0.0;
     // FP64 Stokes work vectors (contiguous: dim velocity comps then p)
     double* V = nullptr;  // (m+1) vectors
-    double* r = nullptr;
     double* w = nullptr;
     double* tmp = nullptr;
     double* xs = nullptr;  // solution copy for the host-fab path
     double* scratch_fc[3] = {nullptr, nullptr, nullptr};
     // reductions
     double* red_partials = nullptr;
+    fhd::GSData gs = {};
     unsigned* red_counter = nullptr;
     double* dscal = nullptr;  // device scalars
     double* hscal = nullptr;  // pinned host mirror
@@ -341,7 +341,8 @@ inline int refuse_reservoirs(const fhd_ctx* c, const char* where) {
 
 constexpr int NSCAL = 256;
 // scalar slots
-constexpr int S_H = 0;        // H column, 1..m+1
+constexpr int S_H = 0;        // H column, 1..m (m <= 60)
+constexpr int S_N2 = 64;      // |u_k|^2 of the Krylov vectors, 0..m
 constexpr int S_NRM = 128;    // norm squares
 constexpr int S_MEAN = 140;   // mean sums
 constexpr int S_Y = 160;      // least-squares y (m <= 64)
@@ -359,7 +360,8 @@ inline RedSlot slot(fhd_ctx* c, int i) {
 }
 
 int precon(fhd_ctx* ctx, CSVec<double> b, SVec<double> x);
-int stokes_apply(fhd_ctx* ctx, CSVec<double> x, CSVec<double> rhs, SVec<double> out, int mode);
+int stokes_apply(fhd_ctx* ctx, CSVec<double> x, CSVec<double> rhs, SVec<double> out, int mode,
+                 const double* inv = nullptr);
 int prepare(fhd_ctx* ctx, const double* const alpha_fc[], const double* beta, const double* const beta_ed[],
             const double* gamma, double theta);
 int stag_mg_solve_dev(fhd_ctx* ctx, double* const phi[], const double* const rhs[]);

@@ -71,21 +71,6 @@ __device__ __forceinline__ void red_finish(double v, RedSlot rs) {
     }
 }
 
-// sum_c w_c * sum_f a_c[f] b_c[f]; weights: 1 for velocity, wp for p
-template <typename TA, typename TB>
-static __global__ void __launch_bounds__(RED_THREADS) k_sdot(i64 n, int ncomp, CSVec<TA> a, CSVec<TB> b, double wlast,
-                                                      RedSlot rs) {
-    double s = 0.0;
-    for (i64 f = blockIdx.x * (i64)blockDim.x + threadIdx.x; f < n; f += (i64)gridDim.x * blockDim.x) {
-        double su = 0.0;
-        for (int c = 0; c < ncomp - 1; c++) su += (double)a.c[c][f] * (double)b.c[c][f];
-        const int c = ncomp - 1;
-        su += wlast * ((double)a.c[c][f] * (double)b.c[c][f]);
-        s += su;
-    }
-    red_finish(s, rs);
-}
-
 // sum_f a[f]
 template <typename T>
 static __global__ void __launch_bounds__(RED_THREADS) k_sum(i64 n, const T* a, RedSlot rs) {
@@ -94,59 +79,188 @@ static __global__ void __launch_bounds__(RED_THREADS) k_sum(i64 n, const T* a, R
     red_finish(s, rs);
 }
 
-// Modified Gram-Schmidt step (gmres.f90:352-378), fused: w -= h*vprev with
-// h read from device memory, then the weighted dot of the updated w with
-// vnext (or with itself when vnext is null).
-static __global__ void __launch_bounds__(RED_THREADS) k_mgs(i64 n, int ncomp, SVec<double> w, CSVec<double> vprev,
-                                                     const double* hprev, CSVec<double> vnext, double wp2,
-                                                     RedSlot rs) {
-    const double h = hprev ? *hprev : 0.0;
-    double s = 0.0;
+// ---------------------------------------------------------------------
+// Orthogonalisation of a new Krylov vector w against i others
+// (gmres.f90:352-389), two passes over the vectors instead of one per
+// vector.  Modified Gram-Schmidt takes h_k = <w - sum_{j<k} h_j v_j, v_k>,
+// that is h_k = <w, v_k> - sum_{j<k} h_j <v_j, v_k>: all products <w, v_k> and
+// the new row of <v_j, v_k> come from one pass (k_gs_dots, whose last block
+// solves for h), and w - sum h_k v_k with its norm from a second
+// (k_gs_update).  The loss of orthogonality stays that of modified
+// Gram-Schmidt, whose coefficients these are.
+//
+// The vectors are kept as computed (u_k, with n2_k = |u_k|^2) rather than
+// scaled to length one: v_k = u_k / |u_k| enters through its coefficients,
+// and the operator scales its result (k_stokes_apply's inv).  So a step moves
+// 2 i + 3 vectors where one pass per vector and the scaling moved 4 i + 3.
+//
+// Bound: DRAM (192^3, five vectors: dots 279 us, update 281 us for 1.6 GB,
+// 5.6 TB/s).  Seven steps of the 192^3 solve with their norms: 5.2 ms one
+// vector at a time with the scaling, 2.7 ms now.  Four resident blocks per SM
+// and all components of an element loaded together keep enough bytes in
+// flight (|w|^2 at 192^3: 97 us with one component after the other, 42 now).
+// ---------------------------------------------------------------------
+constexpr int GS_MAXV = 6;      // vectors per launch
+constexpr int GS_BLOCKS = 592;  // 4 blocks of 256 threads per SM
+constexpr int GS_MAXM = 64;
+
+// device scalars of the orthogonalisation, vector index 0-based
+struct GSData {
+    double* h;        // h_1.. of the current column, at [1 + k]
+    double* n2;       // |u_k|^2
+    double* inv;      // 1 / |u_k|
+    double* coef;     // h_k / |u_k|
+    double* d;        // <w, u_k>
+    double* g;        // <u_{i-1}, u_k>
+    double* gram;     // <v_j, v_k> at [k * GS_MAXM + j], j < k
+    double* partials; // GS_BLOCKS x 2 GS_MAXV
+    unsigned* counter;
+};
+
+// block sums of N values per thread, then over the blocks in block order by
+// the last block; true there, with the sums in out[0 .. N)
+template <int N>
+__device__ __forceinline__ bool red_many(const double (&v)[N], double* partials, unsigned* counter, double* out) {
+    __shared__ double sh[N][RED_THREADS / 32];
+    __shared__ bool last;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = RED_THREADS / 32;
+#pragma unroll
+    for (int q = 0; q < N; q++) {
+        const double s = warp_sum(v[q]);
+        if (lane == 0) sh[q][wid] = s;
+    }
+    __syncthreads();
+    if (threadIdx.x < N) {
+        double s = 0.0;
+#pragma unroll
+        for (int k = 0; k < nw; k++) s += sh[threadIdx.x][k];
+        partials[(size_t)threadIdx.x * GS_BLOCKS + blockIdx.x] = s;
+        __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) last = (atomicAdd(counter, 1u) == gridDim.x - 1);
+    __syncthreads();
+    if (!last) return false;
+    __threadfence();
+    for (int q = wid; q < N; q += nw) {
+        double s = 0.0;
+        for (int b = lane; b < (int)gridDim.x; b += 32) s += __ldcg(partials + (size_t)q * GS_BLOCKS + b);
+        s = warp_sum(s);
+        if (lane == 0) out[q] = s;
+    }
+    if (threadIdx.x == 0) *counter = 0u;
+    __syncthreads();
+    return true;
+}
+
+// weighted |a|^2 (weight 1 for the velocity, wp2 for the pressure); with its
+// inverse root where inv is not null
+template <int NC>
+static __global__ void __launch_bounds__(RED_THREADS, 4) k_norm2(i64 n, CSVec<double> a, double wp2, double* out,
+                                                                 double* inv, double* partials, unsigned* counter) {
+    __shared__ double tot[1];
+    double s[1] = {0.0};
     for (i64 f = blockIdx.x * (i64)blockDim.x + threadIdx.x; f < n; f += (i64)gridDim.x * blockDim.x) {
+        double x[NC];
+#pragma unroll
+        for (int c = 0; c < NC; c++) x[c] = a.c[c][f];
         double su = 0.0;
-        for (int c = 0; c < ncomp; c++) {
-            double x = w.c[c][f];
-            if (hprev) {
-                x = x - vprev.c[c][f] * h;
-                w.c[c][f] = x;
-            }
-            const double y = vnext.c[0] ? vnext.c[c][f] : x;
-            const double t = x * y;
-            su += (c == ncomp - 1) ? wp2 * t : t;
+#pragma unroll
+        for (int c = 0; c < NC - 1; c++) su += x[c] * x[c];
+        su += wp2 * (x[NC - 1] * x[NC - 1]);
+        s[0] += su;
+    }
+    if (!red_many<1>(s, partials, counter, tot) || threadIdx.x) return;
+    *out = tot[0];
+    if (inv) *inv = 1.0 / sqrt(tot[0]);
+}
+
+// <w, u_k> and <u_{i-1}, u_k> for k = k0 .. k0 + NV - 1; the last block of the
+// launch that reaches k = i - 1 solves for h_k
+template <int NC, int NV>
+static __global__ void __launch_bounds__(RED_THREADS, 4) k_gs_dots(i64 n, CSVec<double> w, const double* __restrict__ V,
+                                                                   i64 vstride, int k0, int i, double wp2, GSData G) {
+    __shared__ double tot[2 * NV];
+    double s[2 * NV];
+#pragma unroll
+    for (int q = 0; q < 2 * NV; q++) s[q] = 0.0;
+    const double* __restrict__ ul = V + (i64)(i - 1) * vstride;
+    const double* __restrict__ uk = V + (i64)k0 * vstride;
+    for (i64 f = blockIdx.x * (i64)blockDim.x + threadIdx.x; f < n; f += (i64)gridDim.x * blockDim.x) {
+        double x[NC], l[NC];
+#pragma unroll
+        for (int c = 0; c < NC; c++) {
+            x[c] = w.c[c][f];
+            l[c] = ul[(i64)c * n + f];
         }
-        s += su;
+        x[NC - 1] *= wp2;
+        l[NC - 1] *= wp2;
+#pragma unroll
+        for (int v = 0; v < NV; v++) {
+            double a = 0.0, b = 0.0;
+#pragma unroll
+            for (int c = 0; c < NC; c++) {
+                const double u = uk[v * vstride + (i64)c * n + f];
+                a += x[c] * u;
+                b += l[c] * u;
+            }
+            s[v] += a;
+            s[NV + v] += b;
+        }
     }
-    red_finish(s, rs);
+    if (!red_many<2 * NV>(s, G.partials, G.counter, tot)) return;
+    const int t = threadIdx.x;
+    if (t < NV) {
+        G.d[k0 + t] = tot[t];
+        G.g[k0 + t] = tot[NV + t];
+    }
+    if (k0 + NV < i) return;
+    __syncthreads();
+    // h = (I + L)^-1 <w, v>, L the strictly lower triangle of <v_j, v_k>
+    double* row = G.gram + (size_t)(i - 1) * GS_MAXM;
+    for (int k = t; k < i - 1; k += blockDim.x) row[k] = G.g[k] * G.inv[i - 1] * G.inv[k];
+    __syncthreads();
+    if (t != 0) return;
+    for (int k = 0; k < i; k++) {
+        double h = G.d[k] * G.inv[k];
+        const double* Lk = G.gram + (size_t)k * GS_MAXM;
+        for (int j = 0; j < k; j++) h -= Lk[j] * G.h[1 + j];
+        G.h[1 + k] = h;
+        G.coef[k] = h * G.inv[k];
+    }
 }
 
-// v = w / sqrt(nrm2)  (gmres.f90:380-389 with H(i+1,i) = sqrt(nrm2))
-// (every component of an element is loaded before any is stored, so a
-// thread keeps ncomp loads in flight although v and w may alias)
-static __global__ void __launch_bounds__(256) k_scale_by_norm(i64 n, int ncomp, SVec<double> v, CSVec<double> w,
-                                                       const double* nrm2) {
-    const double h = sqrt(*nrm2);
+// out = w - sum_k coef_k u_k for k = k0 .. k0 + NV - 1, in that order; norm:
+// its |.|^2 and inverse root as those of u_i
+template <int NC, int NV>
+static __global__ void __launch_bounds__(RED_THREADS, 4) k_gs_update(i64 n, CSVec<double> w, SVec<double> out,
+                                                                     const double* __restrict__ V, i64 vstride, int k0,
+                                                                     int i, int norm, double wp2, GSData G) {
+    __shared__ double tot[1];
+    double s[1] = {0.0};
+    double co[NV];
+#pragma unroll
+    for (int v = 0; v < NV; v++) co[v] = G.coef[k0 + v];
+    const double* __restrict__ uk = V + (i64)k0 * vstride;
     for (i64 f = blockIdx.x * (i64)blockDim.x + threadIdx.x; f < n; f += (i64)gridDim.x * blockDim.x) {
-        double a[4];
+        double x[NC];
 #pragma unroll
-        for (int c = 0; c < 4; c++)
-            if (c < ncomp) a[c] = w.c[c][f];
+        for (int c = 0; c < NC; c++) x[c] = w.c[c][f];
 #pragma unroll
-        for (int c = 0; c < 4; c++)
-            if (c < ncomp) v.c[c][f] = a[c] / h;
+        for (int v = 0; v < NV; v++)
+#pragma unroll
+            for (int c = 0; c < NC; c++) x[c] = x[c] - uk[v * vstride + (i64)c * n + f] * co[v];
+        double su = 0.0;
+#pragma unroll
+        for (int c = 0; c < NC; c++) {
+            out.c[c][f] = x[c];
+            su += (c == NC - 1) ? wp2 * (x[c] * x[c]) : x[c] * x[c];
+        }
+        s[0] += su;
     }
-}
-
-// v = w / s (host scalar)
-static __global__ void __launch_bounds__(256) k_scale_div(i64 n, int ncomp, SVec<double> v, CSVec<double> w, double s) {
-    for (i64 f = blockIdx.x * (i64)blockDim.x + threadIdx.x; f < n; f += (i64)gridDim.x * blockDim.x) {
-        double a[4];
-#pragma unroll
-        for (int c = 0; c < 4; c++)
-            if (c < ncomp) a[c] = w.c[c][f];
-#pragma unroll
-        for (int c = 0; c < 4; c++)
-            if (c < ncomp) v.c[c][f] = a[c] / s;
-    }
+    if (!norm || !red_many<1>(s, G.partials, G.counter, tot) || threadIdx.x) return;
+    G.n2[i] = tot[0];
+    G.inv[i] = 1.0 / sqrt(tot[0]);
 }
 
 // x += sum_{it < m} y[it] v_it (update_sol, gmres.f90:495-529; same order)
@@ -207,11 +321,12 @@ static __global__ void __launch_bounds__(256) k_recip(i64 n, T* o, const double*
 // ---------------------------------------------------------------------
 // saddle-point operator, one pass (apply_matrix.f90:117-147):
 //   b_u = (alpha_scale*alpha - L) x_u + G x_p ;  b_p = -D x_u
-// mode 1 returns rhs - A x instead (the GMRES residual, gmres.f90:205-213).
+// mode 1 returns rhs - A x instead (the GMRES residual, gmres.f90:205-213);
+// inv (device scalar, not null in mode 0 only) multiplies A x.
 // ---------------------------------------------------------------------
 template <int DIM, int VISC>
 static __global__ void __launch_bounds__(256) k_stokes_apply(Grid g, StagOp<double> A, CSVec<double> x, CSVec<double> rhs,
-                                                      SVec<double> out, int mode, double dxinv) {
+                                                      SVec<double> out, int mode, double dxinv, const double* inv) {
     CellF P;
     if (!cellf_of_thread(g, P)) return;
     const double* phi[3] = {x.c[0], x.c[1], DIM == 3 ? x.c[2] : nullptr};
@@ -226,11 +341,11 @@ static __global__ void __launch_bounds__(256) k_stokes_apply(Grid g, StagOp<doub
         double L = stag_lface_c<double, DIM, VISC>(c, A, phi, P, dg);
         const double gp = (pc - ld(p, P.id(-dx_, -dy_, -dz_))) * dxinv;
         L = L + gp;
-        out.c[c][f] = mode ? ld(rhs.c[c], f) - L : L;
+        out.c[c][f] = mode ? ld(rhs.c[c], f) - L : inv ? L * *inv : L;
         div += (ld(phi[c], P.id(dx_, dy_, dz_)) - ld(phi[c], f)) * dxinv;
     }
     const double bp = div * -1.0;
-    out.c[DIM][f] = mode ? ld(rhs.c[DIM], f) - bp : bp;
+    out.c[DIM][f] = mode ? ld(rhs.c[DIM], f) - bp : inv ? bp * *inv : bp;
 }
 
 // the same with gmres_spatial_order = 4 (apply_matrix.f90:124-135): the
@@ -244,7 +359,7 @@ static __global__ void __launch_bounds__(256) k_stokes_apply(Grid g, StagOp<doub
 template <int DIM>
 static __global__ void __launch_bounds__(256) k_stokes_apply4(Grid g, StagOp<double> A, CSVec<double> x,
                                                               CSVec<double> rhs, SVec<double> out, int mode,
-                                                              double dxinv, double t1, double t2) {
+                                                              double dxinv, double t1, double t2, const double* inv) {
     Cell P;
     if (!cell_of_thread(g, P)) return;
     const double b = ld(A.beta, 0);
@@ -272,11 +387,11 @@ static __global__ void __launch_bounds__(256) k_stokes_apply4(Grid g, StagOp<dou
                            ld(p, P.id(-2 * e0, -2 * e1, -2 * e2))) *
                           t1;
         L = L + gp;
-        out.c[c][f] = mode ? ld(rhs.c[c], f) - L : L;
+        out.c[c][f] = mode ? ld(rhs.c[c], f) - L : inv ? L * *inv : L;
         div += (ld(u, P.id(e0, e1, e2)) - ld(u, f)) * dxinv;
     }
     const double bp = div * -1.0;
-    out.c[DIM][f] = mode ? ld(rhs.c[DIM], f) - bp : bp;
+    out.c[DIM][f] = mode ? ld(rhs.c[DIM], f) - bp : inv ? bp * *inv : bp;
 }
 
 // mac_rhs = D x_u + b_p  (apply_precon.f90:118-123)

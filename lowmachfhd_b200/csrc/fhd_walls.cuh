@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(256) k_zero_walls(Grid g, Walls W, T* u0, T* u
 template <int DIM, int VISC>
 static __global__ void __launch_bounds__(256) k_stokes_apply_w(Grid g, Walls W, StagOp<double> A, CSVec<double> x,
                                                                CSVec<double> rhs, SVec<double> out, int mode,
-                                                               double dxinv) {
+                                                               double dxinv, const double* inv) {
     Cell P;
     if (!cell_of_thread(g, P)) return;
     const double* phi[3] = {x.c[0], x.c[1], DIM == 3 ? x.c[2] : nullptr};
@@ -208,11 +208,11 @@ static __global__ void __launch_bounds__(256) k_stokes_apply_w(Grid g, Walls W, 
             const double gp = (pc - ld(p, P.id(-dx_, -dy_, -dz_))) * dxinv;
             L = L + gp;
         }
-        out.c[c][f] = mode ? ld(rhs.c[c], f) - L : L;
+        out.c[c][f] = mode ? ld(rhs.c[c], f) - L : inv ? L * *inv : L;
         div += (ld(phi[c], P.id(dx_, dy_, dz_)) - ld(phi[c], f)) * dxinv;
     }
     const double bp = div * -1.0;
-    out.c[DIM][f] = mode ? ld(rhs.c[DIM], f) - bp : bp;
+    out.c[DIM][f] = mode ? ld(rhs.c[DIM], f) - bp : inv ? bp * *inv : bp;
 }
 
 // host dispatch of the wall kernels on the context's visc_type (1, 2 or 3)
