@@ -28,45 +28,55 @@ struct StochArgs {
 // scaled random stress at a cell (component c) or on an edge (edge set e,
 // component comp): variance * (sum_r w_r W_r) * sqrt(eta T)
 // (stochastic_m_fluxdiv.f90:115-125, 137, 280-361)
-template <typename T>
+// NR > 0: n_rngs as a constant, so that the loads of all fields and stresses
+// are in flight together
+template <typename T, int NR = 0>
 __device__ __forceinline__ T stoch_cc(const StochArgs& a, int dim, int c, i64 f) {
     T s = T(0);
-    for (int r = 0; r < a.n_rngs; r++) s = s + (T)a.wts[r] * (T)ld(a.Wcc[r * dim + c], f);
+#pragma unroll
+    for (int r = 0; r < (NR ? NR : a.n_rngs); r++) s = s + (T)a.wts[r] * (T)ld(a.Wcc[r * dim + c], f);
     return ((T)a.variance * s) * (T)sqrt((T)ld(a.eta, f) * (T)ld(a.T, f));
 }
-template <typename T>
+template <typename T, int NR = 0>
 __device__ __forceinline__ T stoch_ed(const StochArgs& a, int nE, int e, int comp, i64 f) {
     T s = T(0);
-    for (int r = 0; r < a.n_rngs; r++) s = s + (T)a.wts[r] * (T)ld(a.Wed[r * 2 * nE + 2 * e + comp], f);
+#pragma unroll
+    for (int r = 0; r < (NR ? NR : a.n_rngs); r++) s = s + (T)a.wts[r] * (T)ld(a.Wed[r * 2 * nE + 2 * e + comp], f);
     return ((T)a.variance * s) * (T)sqrt((T)ld(a.eta_ed[e], f) * (T)ld(a.T_ed[e], f));
 }
 
 // divergence of the scaled random stress onto the faces (stoch_m_force_2d /
 // _3d, stochastic_m_fluxdiv.f90:453-600), overwrite or increment.
 // T is the arithmetic precision (double, or float in the mixed mode).
-template <typename T, int DIM>
+// NR: n_rngs of 1 or 2 as a constant, else 0.  A face reads up to 54 values;
+// what bounds it is having them in flight: with the loop over the noise fields
+// at run time each stress waited for its own loads (192^3, one field: 380 us),
+// unrolled 233 us, 4.2 TB/s for 0.98 GB, the conversions to FP32 taking three
+// quarters of their pipe.  (A march in z with 17 loads per cell through shared
+// memory took 334 us: too few warps for its chain of root and barrier.)
+template <typename T, int DIM, int NR>
 __global__ void __launch_bounds__(256) k_stoch_m(Grid g, StochArgs a, double* o0, double* o1, double* o2,
                                                  int increment) {
-    Cell P;
-    if (!cell_of_thread(g, P)) return;
+    CellF P;
+    if (!cellf_of_thread(g, P)) return;
     const i64 f = P.id(0, 0, 0);
     const T dxi = (T)a.dxinv;
     T dv[3];
     if constexpr (DIM == 2) {
-        dv[0] = (stoch_cc<T>(a, 2, 0, f) - stoch_cc<T>(a, 2, 0, P.id(-1, 0, 0))) * dxi +
-                (stoch_ed<T>(a, 1, 0, 0, P.id(0, 1, 0)) - stoch_ed<T>(a, 1, 0, 0, f)) * dxi;
-        dv[1] = (stoch_ed<T>(a, 1, 0, 1, P.id(1, 0, 0)) - stoch_ed<T>(a, 1, 0, 1, f)) * dxi +
-                (stoch_cc<T>(a, 2, 1, f) - stoch_cc<T>(a, 2, 1, P.id(0, -1, 0))) * dxi;
+        dv[0] = (stoch_cc<T, NR>(a, 2, 0, f) - stoch_cc<T, NR>(a, 2, 0, P.id(-1, 0, 0))) * dxi +
+                (stoch_ed<T, NR>(a, 1, 0, 0, P.id(0, 1, 0)) - stoch_ed<T, NR>(a, 1, 0, 0, f)) * dxi;
+        dv[1] = (stoch_ed<T, NR>(a, 1, 0, 1, P.id(1, 0, 0)) - stoch_ed<T, NR>(a, 1, 0, 1, f)) * dxi +
+                (stoch_cc<T, NR>(a, 2, 1, f) - stoch_cc<T, NR>(a, 2, 1, P.id(0, -1, 0))) * dxi;
     } else {
-        dv[0] = (stoch_cc<T>(a, 3, 0, f) - stoch_cc<T>(a, 3, 0, P.id(-1, 0, 0))) * dxi +
-                (stoch_ed<T>(a, 3, 0, 0, P.id(0, 1, 0)) - stoch_ed<T>(a, 3, 0, 0, f)) * dxi +
-                (stoch_ed<T>(a, 3, 1, 0, P.id(0, 0, 1)) - stoch_ed<T>(a, 3, 1, 0, f)) * dxi;
-        dv[1] = (stoch_ed<T>(a, 3, 0, 1, P.id(1, 0, 0)) - stoch_ed<T>(a, 3, 0, 1, f)) * dxi +
-                (stoch_cc<T>(a, 3, 1, f) - stoch_cc<T>(a, 3, 1, P.id(0, -1, 0))) * dxi +
-                (stoch_ed<T>(a, 3, 2, 0, P.id(0, 0, 1)) - stoch_ed<T>(a, 3, 2, 0, f)) * dxi;
-        dv[2] = (stoch_ed<T>(a, 3, 1, 1, P.id(1, 0, 0)) - stoch_ed<T>(a, 3, 1, 1, f)) * dxi +
-                (stoch_ed<T>(a, 3, 2, 1, P.id(0, 1, 0)) - stoch_ed<T>(a, 3, 2, 1, f)) * dxi +
-                (stoch_cc<T>(a, 3, 2, f) - stoch_cc<T>(a, 3, 2, P.id(0, 0, -1))) * dxi;
+        dv[0] = (stoch_cc<T, NR>(a, 3, 0, f) - stoch_cc<T, NR>(a, 3, 0, P.id(-1, 0, 0))) * dxi +
+                (stoch_ed<T, NR>(a, 3, 0, 0, P.id(0, 1, 0)) - stoch_ed<T, NR>(a, 3, 0, 0, f)) * dxi +
+                (stoch_ed<T, NR>(a, 3, 1, 0, P.id(0, 0, 1)) - stoch_ed<T, NR>(a, 3, 1, 0, f)) * dxi;
+        dv[1] = (stoch_ed<T, NR>(a, 3, 0, 1, P.id(1, 0, 0)) - stoch_ed<T, NR>(a, 3, 0, 1, f)) * dxi +
+                (stoch_cc<T, NR>(a, 3, 1, f) - stoch_cc<T, NR>(a, 3, 1, P.id(0, -1, 0))) * dxi +
+                (stoch_ed<T, NR>(a, 3, 2, 0, P.id(0, 0, 1)) - stoch_ed<T, NR>(a, 3, 2, 0, f)) * dxi;
+        dv[2] = (stoch_ed<T, NR>(a, 3, 1, 1, P.id(1, 0, 0)) - stoch_ed<T, NR>(a, 3, 1, 1, f)) * dxi +
+                (stoch_ed<T, NR>(a, 3, 2, 1, P.id(0, 1, 0)) - stoch_ed<T, NR>(a, 3, 2, 1, f)) * dxi +
+                (stoch_cc<T, NR>(a, 3, 2, f) - stoch_cc<T, NR>(a, 3, 2, P.id(0, 0, -1))) * dxi;
     }
     double* o[3] = {o0, o1, o2};
 #pragma unroll
@@ -330,15 +340,21 @@ int stoch_launch(fhd_ctx* ctx, const fhd_stoch_params* sp, double* const force[]
         FHD_CUDA_TRY(cudaPeekAtLastError());
         return 0;
     }
-    with_dim(dim, [&](auto D) {
-        constexpr int DIM = decltype(D)::value;
-        if (mixed)
-            k_stoch_m<float, DIM><<<cell_grid(g), cell_block(), 0, ctx->stream>>>(g, a, force[0], force[1], f2,
-                                                                                increment);
-        else
-            k_stoch_m<double, DIM><<<cell_grid(g), cell_block(), 0, ctx->stream>>>(g, a, force[0], force[1], f2,
-                                                                                 increment);
-    });
+    auto run = [&](auto Nr) {
+        constexpr int NR = decltype(Nr)::value;
+        with_dim(dim, [&](auto D) {
+            constexpr int DIM = decltype(D)::value;
+            if (mixed)
+                k_stoch_m<float, DIM, NR><<<cell_grid(g), cell_block(), 0, ctx->stream>>>(g, a, force[0], force[1], f2,
+                                                                                        increment);
+            else
+                k_stoch_m<double, DIM, NR><<<cell_grid(g), cell_block(), 0, ctx->stream>>>(g, a, force[0], force[1],
+                                                                                         f2, increment);
+        });
+    };
+    if (n_rngs == 1) run(std::integral_constant<int, 1>());
+    else if (n_rngs == 2) run(std::integral_constant<int, 2>());
+    else run(std::integral_constant<int, 0>());
     ctx->launches++;
     FHD_CUDA_TRY(cudaPeekAtLastError());
     return 0;
