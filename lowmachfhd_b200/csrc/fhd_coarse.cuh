@@ -46,7 +46,7 @@
 #pragma once
 #include <type_traits>
 
-#include "fhd_kernels.cuh"
+#include "fhd_walls.cuh"
 
 namespace fhd {
 
@@ -136,9 +136,12 @@ struct CSNear {
 };
 
 // The x-pairs of a split level, dealt to its first nt threads: thread t takes
-// pair t % np of every RP-th row.  Worked out once per level.
+// pair t % np of every RP-th row.  Worked out once per level.  With walls
+// (WALL, set_walls) a neighbour behind a wall is -1.
+template <bool WALL = false>
 struct CSPairs {
     int np, ny, nz, nh, nt;
+    bool wx = false, wy = false, wz = false;
     int h0, j0, k0, dj, dk, RP;
     bool on;
     __device__ __forceinline__ void set(const Grid& g) {
@@ -152,13 +155,19 @@ struct CSPairs {
         cs_divmod(r, ny, k0, j0);
         cs_divmod(RP, ny, dk, dj);
     }
+    __device__ __forceinline__ void set_walls(const Walls& W) {
+        wx = W.lo[0] != 0;
+        wy = W.lo[1] != 0;
+        wz = W.lo[2] != 0;
+    }
     // f(pair, its row's parity and first pair, those of the rows below and
     // above in y and z)
     template <class F>
     __device__ __forceinline__ void row(int h, int j, int k, F&& f) const {
         const int nl = np * ny, b = np * j + nl * k;
-        f(h, j + k, b, j == 0 ? b + nl - np : b - np, j == ny - 1 ? b - nl + np : b + np,
-          k == 0 ? b + nl * (nz - 1) : b - nl, k == nz - 1 ? b - nl * (nz - 1) : b + nl);
+        const bool y_ = WALL && wy, z_ = WALL && wz;
+        f(h, j + k, b, j == 0 ? (y_ ? -1 : b + nl - np) : b - np, j == ny - 1 ? (y_ ? -1 : b - nl + np) : b + np,
+          k == 0 ? (z_ ? -1 : b + nl * (nz - 1)) : b - nl, k == nz - 1 ? (z_ ? -1 : b - nl * (nz - 1)) : b + nl);
     }
     template <class F>
     __device__ __forceinline__ void each(F&& f) const {
@@ -182,8 +191,9 @@ struct CSPairs {
     // the x neighbour in the next pair of the row's cell of colour col: to
     // the left of an even cell, to the right of an odd one
     __device__ __forceinline__ int across(int h, int s, int col) const {
-        if ((s ^ col) & 1) return h + 1 == np ? 0 : h + 1;
-        return h == 0 ? np - 1 : h - 1;
+        const bool x_ = WALL && wx;
+        if ((s ^ col) & 1) return h + 1 == np ? (x_ ? -1 : 0) : h + 1;
+        return h == 0 ? (x_ ? -1 : np - 1) : h - 1;
     }
 };
 
@@ -205,6 +215,7 @@ struct StagCoarseArgs {
     T omega;
     T* phi[3];          // level-0 unknowns in global memory (in/out)
     const T* rhs[3];    // level-0 right-hand side
+    Walls walls;        // (WALL instantiations)
     Grid g[CS_MAXL];
     StagOp<T> A[CS_MAXL];
     int off[CS_MAXL];   // shared-memory element offset of each level
@@ -394,8 +405,8 @@ struct CSLev {
 };
 
 // the diagonals of a split level into its scratch
-template <typename T, int DIM>
-__device__ __forceinline__ void cs_split_diag(const CSPairs& Q, const CSVisc1<T, DIM>& U, const StagOp<T>& A,
+template <typename T, int DIM, class Pairs>
+__device__ __forceinline__ void cs_split_diag(const Pairs& Q, const CSVisc1<T, DIM>& U, const StagOp<T>& A,
                                               const CSLev<T>& V) {
     Q.each([&](int h, int s, int b, int, int, int, int) {
         const int p = b + h, r = s & 1;
@@ -407,80 +418,122 @@ __device__ __forceinline__ void cs_split_diag(const CSPairs& Q, const CSVisc1<T,
     });
 }
 
-// f(element, neighbour pair sums by component) of the cells of colour col
-template <typename T, int DIM, class F>
-__device__ __forceinline__ void cs_split_cells(const CSPairs& Q, const T* ph, int col, F&& f) {
+// value of component c behind a wall of direction d and sign sg: zero normal
+// to it, the face's own value v or its negative along it (wall_vel)
+template <typename T>
+__device__ __forceinline__ T cs_behind(int c, int d, int sg, T v) {
+    return c == d ? T(0) : (sg < 0 ? -v : v);
+}
+
+// f(element, neighbour pair sums by component, components on a wall face) of
+// the cells of colour col
+template <typename T, int DIM, bool WALL, class F>
+__device__ __forceinline__ void cs_split_cells(const CSPairs<WALL>& Q, const Walls& W, const T* ph, int col, F&& f) {
     const int own = (col ? Q.nh : 0) * DIM;
     const T* O = ph + (col ? 0 : Q.nh) * DIM;
     Q.each([&](int h, int s, int b, int ym, int yp, int zm, int zp) {
-        const T *o = O + (b + h) * DIM, *ox = O + (b + Q.across(h, s, col)) * DIM, *op = O + (yp + h) * DIM,
-                *om = O + (ym + h) * DIM, *oq = O + (zp + h) * DIM, *on = O + (zm + h) * DIM;
+        const int hx = Q.across(h, s, col), e = own + (b + h) * DIM;
         T xs[DIM], ys[DIM], zs[DIM];
+        if constexpr (WALL) {
+            const bool odd = (s ^ col) & 1;
+            const int ax = hx < 0 ? -1 : b + hx, ap = yp < 0 ? -1 : yp + h, am = ym < 0 ? -1 : ym + h,
+                      aq = zp < 0 ? -1 : zp + h, an = zm < 0 ? -1 : zm + h;
+            const int on = (Q.wx && !odd && h == 0 ? 1 : 0) | (ym < 0 ? 2 : 0) | (zm < 0 ? 4 : 0);
 #pragma unroll
-        for (int c = 0; c < DIM; c++) {
-            xs[c] = o[c] + ox[c];
-            ys[c] = op[c] + om[c];
-            zs[c] = DIM == 3 ? oq[c] + on[c] : T(0);
+            for (int c = 0; c < DIM; c++) {
+                const T v = ph[e + c];
+                auto at = [&](int a, int d, int sg) { return a < 0 ? cs_behind(c, d, sg, v) : O[a * DIM + c]; };
+                xs[c] = O[(b + h) * DIM + c] + at(ax, 0, odd ? W.hi[0] : W.lo[0]);
+                ys[c] = at(ap, 1, W.hi[1]) + at(am, 1, W.lo[1]);
+                zs[c] = DIM == 3 ? at(aq, 2, W.hi[2]) + at(an, 2, W.lo[2]) : T(0);
+            }
+            f(e, xs, ys, zs, on);
+        } else {
+            const T *o = O + (b + h) * DIM, *ox = O + (b + hx) * DIM, *op = O + (yp + h) * DIM,
+                    *om = O + (ym + h) * DIM, *oq = O + (zp + h) * DIM, *on = O + (zm + h) * DIM;
+#pragma unroll
+            for (int c = 0; c < DIM; c++) {
+                xs[c] = o[c] + ox[c];
+                ys[c] = op[c] + om[c];
+                zs[c] = DIM == 3 ? oq[c] + on[c] : T(0);
+            }
+            f(e, xs, ys, zs, 0);
         }
-        f(own + (b + h) * DIM, xs, ys, zs);
     });
 }
 
 // count smooths of a split level, its diagonals in the scratch
-template <typename T, int DIM>
-__device__ __forceinline__ void cs_split_smooths(const CSPairs& Q, const CSVisc1<T, DIM>& U, const CSLev<T>& V,
-                                                 int count) {
+template <typename T, int DIM, bool WALL>
+__device__ __forceinline__ void cs_split_smooths(const CSPairs<WALL>& Q, const Walls& W, const CSVisc1<T, DIM>& U,
+                                                 const CSLev<T>& V, int count) {
     for (int m = 0; m < 2 * count; m++) {
-        cs_split_cells<T, DIM>(Q, V.ph, m & 1, [&](int e, const T* xs, const T* ys, const T* zs) {
+        cs_split_cells<T, DIM, WALL>(Q, W, V.ph, m & 1, [&](int e, const T* xs, const T* ys, const T* zs, int on) {
             T nv[DIM];
 #pragma unroll
             for (int c = 0; c < DIM; c++)
                 nv[c] = U.update(c, V.ph[e + c], xs[c], ys[c], zs[c], V.rh[e + c], V.tm[e + c]);
 #pragma unroll
-            for (int c = 0; c < DIM; c++) V.ph[e + c] = nv[c];
+            for (int c = 0; c < DIM; c++)
+                if (!(on >> c & 1)) V.ph[e + c] = nv[c];
         });
         cs_bar(Q.nt);
     }
 }
 
-// residual of a split level over its diagonals
-template <typename T, int DIM>
-__device__ __forceinline__ void cs_split_residual(const CSPairs& Q, const CSVisc1<T, DIM>& U, const CSLev<T>& V) {
+// residual of a split level over its diagonals, zero on wall faces
+template <typename T, int DIM, bool WALL>
+__device__ __forceinline__ void cs_split_residual(const CSPairs<WALL>& Q, const Walls& W, const CSVisc1<T, DIM>& U,
+                                                  const CSLev<T>& V) {
     for (int col = 0; col < 2; col++)
-        cs_split_cells<T, DIM>(Q, V.ph, col, [&](int e, const T* xs, const T* ys, const T* zs) {
+        cs_split_cells<T, DIM, WALL>(Q, W, V.ph, col, [&](int e, const T* xs, const T* ys, const T* zs, int on) {
             T nv[DIM];
 #pragma unroll
             for (int c = 0; c < DIM; c++)
                 nv[c] = U.resid(c, V.ph[e + c], xs[c], ys[c], zs[c], V.rh[e + c], V.tm[e + c]);
 #pragma unroll
-            for (int c = 0; c < DIM; c++) V.tm[e + c] = nv[c];
+            for (int c = 0; c < DIM; c++) V.tm[e + c] = (on >> c & 1) ? T(0) : nv[c];
         });
 }
 
 // smooths of an odd level: each colour of every component from one buffer
 // into the other (an even number of times)
-template <typename T, int DIM>
-__device__ __forceinline__ void cs_odd_smooths(const Grid& g, const CSVisc1<T, DIM>& U, const StagOp<T>& A,
-                                               const CSLev<T>& V, int count, int nt) {
+template <typename T, int DIM, bool WALL>
+__device__ __forceinline__ void cs_odd_smooths(const Grid& g, const Walls& W, const CSVisc1<T, DIM>& U,
+                                               const StagOp<T>& A, const CSLev<T>& V, int count, int nt) {
     const int nc = (int)g.nc;
     T *x = V.ph, *y = V.tm;
     for (int s = 0; s < 2 * count; s++) {
         for (int f0 = threadIdx.x; f0 < nc; f0 += nt) {
-            int i, j, k;
-            cs_ijk(g, f0, i, j, k);
+            int q[3];
+            cs_ijk(g, f0, q[0], q[1], q[2]);
             T nv[DIM];
 #pragma unroll
             for (int c = 0; c < DIM; c++) nv[c] = x[f0 * DIM + c];
-            if (((i + j + k) & 1) == (s & 1)) {
+            if (((q[0] + q[1] + q[2]) & 1) == (s & 1)) {
                 CellF P;
-                P.set(g, i, j, k);
+                P.set(g, q[0], q[1], q[2]);
                 const int xm = (int)P.id(-1, 0, 0), xp = (int)P.id(1, 0, 0), ym = (int)P.id(0, -1, 0),
                           yp = (int)P.id(0, 1, 0), zm = (int)P.id(0, 0, -1), zp = (int)P.id(0, 0, 1);
 #pragma unroll
                 for (int c = 0; c < DIM; c++) {
-                    const T zs = DIM == 3 ? x[zp * DIM + c] + x[zm * DIM + c] : T(0);
-                    nv[c] = U.update(c, nv[c], x[xp * DIM + c] + x[xm * DIM + c], x[yp * DIM + c] + x[ym * DIM + c],
-                                     zs, V.rh[f0 * DIM + c], U.as * ld(A.alpha[c], f0) + U.bd);
+                    const T v = nv[c];
+                    T xs, ys, zs = T(0);
+                    if constexpr (WALL) {
+                        if (W.lo[c] != 0 && q[c] == 0) continue;  // on the wall
+                        auto pair = [&](int d, int lo, int hi) {
+                            const bool w = W.lo[d] != 0;
+                            return (w && q[d] == g.n[d] - 1 ? cs_behind(c, d, W.hi[d], v) : x[hi * DIM + c]) +
+                                   (w && q[d] == 0 ? cs_behind(c, d, W.lo[d], v) : x[lo * DIM + c]);
+                        };
+                        xs = pair(0, xm, xp);
+                        ys = pair(1, ym, yp);
+                        if (DIM == 3) zs = pair(2, zm, zp);
+                    } else {
+                        xs = x[xp * DIM + c] + x[xm * DIM + c];
+                        ys = x[yp * DIM + c] + x[ym * DIM + c];
+                        if (DIM == 3) zs = x[zp * DIM + c] + x[zm * DIM + c];
+                    }
+                    nv[c] = U.update(c, v, xs, ys, zs, V.rh[f0 * DIM + c], U.as * ld(A.alpha[c], f0) + U.bd);
                 }
             }
 #pragma unroll
@@ -509,8 +562,11 @@ __device__ __forceinline__ StagOp<T> cs_op(const StagCoarseArgs<T>& a, int m) {
 
 // the coarse end of one staggered V-cycle in the calling CTA (shared memory
 // from the dynamic allocation); also run per box by the batched solver
-template <typename T, int DIM, int VISC>
+// (WALL: visc_type 1 with domain walls)
+template <typename T, int DIM, int VISC, bool WALL = false>
 __device__ __forceinline__ void stag_coarse_run(const StagCoarseArgs<T>& a) {
+    static_assert(!WALL || VISC == 1, "walls: visc_type 1");
+    const Walls& W = a.walls;
     extern __shared__ __align__(16) unsigned char cs_smem[];
     T* S = reinterpret_cast<T*>(cs_smem);
     const int nt = blockDim.x;
@@ -536,16 +592,17 @@ __device__ __forceinline__ void stag_coarse_run(const StagCoarseArgs<T>& a) {
                 CSVisc1<T, DIM> U;
                 U.set(A, a.omega);
                 if (cs_all_even(g)) {
-                    CSPairs Q;
+                    CSPairs<WALL> Q;
                     Q.set(g);
+                    if (WALL) Q.set_walls(W);
                     if ((int)threadIdx.x < Q.nt) {
                         cs_split_diag<T, DIM>(Q, U, A, V);  // (each thread reads the ones it wrote)
-                        cs_split_smooths<T, DIM>(Q, U, V, count);
-                        if (res) cs_split_residual<T, DIM>(Q, U, V);
+                        cs_split_smooths<T, DIM, WALL>(Q, W, U, V, count);
+                        if (res) cs_split_residual<T, DIM, WALL>(Q, W, U, V);
                     }
                 } else {
                     const int na = (int)g.nc >= nt ? nt : ((int)g.nc + 31) & ~31;
-                    if ((int)threadIdx.x < na) cs_odd_smooths<T, DIM>(g, U, A, V, count, na);
+                    if ((int)threadIdx.x < na) cs_odd_smooths<T, DIM, WALL>(g, W, U, A, V, count, na);
                 }
                 __syncthreads();
                 return;
@@ -600,8 +657,31 @@ __device__ __forceinline__ void stag_coarse_run(const StagCoarseArgs<T>& a) {
     for (int m = a.nlev - 2; m >= 0; m--) {
         const CSIdx X = index(m), Y = index(m + 1);
         T* F = arr(m, 0);
-        const T* W = arr(m + 1, 0);
+        const T* Cu = arr(m + 1, 0);
         const int cf = cs(m), cc = cs(m + 1);
+        // the coarse value of component c at an offset, under the wall rules
+        // (wall_vel)
+        auto coarse = [&](const CSNear<DIM>& H, int qi, int qj, int qk, int c, int o, int pa, int pb) {
+            if constexpr (WALL) {
+                int off[3] = {0, 0, 0};
+                off[c] += o;
+                off[c == 0 ? 1 : 0] += pa;
+                if (DIM == 3) off[c == 2 ? 1 : 2] += pb;
+                T sg = T(1);
+#pragma unroll
+                for (int d = 0; d < DIM; d++) {
+                    const int at = (d == 0 ? qi : d == 1 ? qj : qk) + off[d];
+                    const bool lo = at < 0, hi = at >= a.g[m + 1].n[d];
+                    if (W.lo[d] == 0 || (!lo && !hi)) continue;
+                    off[d] = 0;
+                    if (d == c) return T(0);
+                    if ((lo ? W.lo[d] : W.hi[d]) < 0) sg = -sg;
+                }
+                return sg * Cu[H.at(off[0], off[1], off[2]) * es + c * cc];
+            } else {
+                return Cu[H.comp(c, o, pa, pb) * es + c * cc];
+            }
+        };
         for (int q = threadIdx.x; q < (int)a.g[m + 1].nc; q += nt) {
             int qi, qj, qk;
             cs_ijk(a.g[m + 1], q, qi, qj, qk);
@@ -616,7 +696,7 @@ __device__ __forceinline__ void stag_coarse_run(const StagCoarseArgs<T>& a) {
                     for (int pa = -1; pa <= 1; pa++)
 #pragma unroll
                         for (int pb = -1; pb <= 1; pb++)
-                            cv[o][pa + 1][pb + 1] = (DIM == 3 || pb == 0) ? W[H.comp(c, o, pa, pb) * es + c * cc] : T(0);
+                            cv[o][pa + 1][pb + 1] = (DIM == 3 || pb == 0) ? coarse(H, qi, qj, qk, c, o, pa, pb) : T(0);
 #pragma unroll
                 for (int pz = 0; pz < (DIM == 3 ? 2 : 1); pz++)
 #pragma unroll
@@ -629,7 +709,10 @@ __device__ __forceinline__ void stag_coarse_run(const StagCoarseArgs<T>& a) {
                             const int ob = (DIM == 3) ? (I[c == 2 ? 1 : 2] ? 1 : -1) : 0;
                             T* v = F + (r + (X.split ? qi : 2 * qi + px) + (((px + py + pz) & 1) ? X.co : 0)) * es +
                                    c * cf;
-                            *v = *v + stag_prolong_expr<T, DIM>(I[c] == 0, oa, ob, [&](int o, int pa, int pb) {
+                            const bool on = WALL && W.lo[c] != 0 && I[c] == 0 &&
+                                            (c == 0 ? qi : c == 1 ? qj : qk) == 0;
+                            if (!on)
+                                *v = *v + stag_prolong_expr<T, DIM>(I[c] == 0, oa, ob, [&](int o, int pa, int pb) {
                                      return cv[o][pa + 1][pb + 1];
                                  });
                         }
@@ -652,9 +735,9 @@ __device__ __forceinline__ void stag_coarse_run(const StagCoarseArgs<T>& a) {
     }
 }
 
-template <typename T, int DIM, int VISC>
+template <typename T, int DIM, int VISC, bool WALL = false>
 __global__ void __launch_bounds__(CS_THREADS) k_stag_coarse(const __grid_constant__ StagCoarseArgs<T> a) {
-    stag_coarse_run<T, DIM, VISC>(a);
+    stag_coarse_run<T, DIM, VISC, WALL>(a);
 }
 
 // ---------------------------------------------------------------------
@@ -721,7 +804,7 @@ struct CSCC {
 // D a G phi and its diagonal at the cell of colour COL in pair h of a row
 // (cc_lap_acc's expression; s: the parity of the row)
 template <typename T, int DIM, int CF>
-__device__ __forceinline__ T cs_cc_lap(const CSPairs& Q, const CCOp<T>& A, const CSCC<T>& V, int col, int h, int s,
+__device__ __forceinline__ T cs_cc_lap(const CSPairs<>& Q, const CCOp<T>& A, const CSCC<T>& V, int col, int h, int s,
                                        int b, int ym, int yp, int zm, int zp, T v, T& diag) {
     const bool odd = (s ^ col) & 1;  // the pair's cell of odd i
     const int hp = odd ? (h + 1 == Q.np ? 0 : h + 1) : h, hm = odd ? h : (h == 0 ? Q.np - 1 : h - 1);
@@ -748,7 +831,7 @@ __device__ __forceinline__ T cs_cc_lap(const CSPairs& Q, const CCOp<T>& A, const
 }
 
 template <typename T, int DIM, int CF>
-__device__ __forceinline__ void cs_cc_split_smooths(const CSPairs& Q, const CCOp<T>& A, const CSCC<T>& V, int count) {
+__device__ __forceinline__ void cs_cc_split_smooths(const CSPairs<>& Q, const CCOp<T>& A, const CSCC<T>& V, int count) {
     auto sweep = [&](auto Col) {
         constexpr int col = decltype(Col)::value;
         Q.each([&](int h, int s, int b, int ym, int yp, int zm, int zp) {
@@ -769,7 +852,7 @@ __device__ __forceinline__ void cs_cc_split_smooths(const CSPairs& Q, const CCOp
 // residual of a split level averaged over the 2^dim children of each coarse
 // cell (cc_resid_avg)
 template <typename T, int DIM, int CF>
-__device__ __forceinline__ void cs_cc_split_restrict(const CSPairs& Q, const CCOp<T>& A, const CSCC<T>& V,
+__device__ __forceinline__ void cs_cc_split_restrict(const CSPairs<>& Q, const CCOp<T>& A, const CSCC<T>& V,
                                                      const Grid& gc, const CSIdx& Y, const CSCC<T>& W) {
     for (int q = threadIdx.x; q < (int)gc.nc; q += blockDim.x) {
         int qi, qj, qk;
@@ -868,7 +951,7 @@ __device__ __forceinline__ void cc_coarse_run(const CCCoarseArgs<T>& a) {
         with_coef(m, [&](auto Cf) {
             constexpr int CF = decltype(Cf)::value;
             if (cs_all_even(a.g[m])) {
-                CSPairs Q;
+                CSPairs<> Q;
                 Q.set(a.g[m]);
                 if ((int)threadIdx.x < Q.nt) cs_cc_split_smooths<T, DIM, CF>(Q, A, V, count);
             } else {
@@ -908,7 +991,7 @@ __device__ __forceinline__ void cc_coarse_run(const CCCoarseArgs<T>& a) {
     for (int m = 0; m + 1 < a.nlev; m++) {
         smooths(m, a.n_down);
         with_coef(m, [&](auto Cf) {
-            CSPairs Q;
+            CSPairs<> Q;
             Q.set(a.g[m]);
             cs_cc_split_restrict<T, DIM, decltype(Cf)::value>(Q, a.A[m], level(m), a.g[m + 1], idx(m + 1),
                                                              level(m + 1));

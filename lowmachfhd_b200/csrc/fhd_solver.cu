@@ -727,11 +727,28 @@ template <typename T>
 static int stag_smooths(fhd_ctx* ctx, StagLevel<T>& L, int count, int zero = 0, bool home = true) {
     const int dim = ctx->dim;
     if (ctx->has_walls) {
-        // the colours of the reference's smoother, each as Lphi and the
-        // diagonal of its faces, then the update (the wall faces stay zero)
         const StagOp<T> A = L.op();
         const T omega = (T)ctx->p.stag_mg_omega;
         int rc = 0;
+        bool even = true;  // in the periodic directions
+        for (int d = 0; d < dim; d++) even = even && (ctx->walls.lo[d] != 0 || !(L.g.n[d] & 1));
+        if (even) {
+            const dim3 blk = cell_block(), grd(((L.g.n[0] + 1) / 2 + blk.x - 1) / blk.x, (L.g.n[1] + blk.y - 1) / blk.y,
+                                               L.g.n[2]);
+            for (int m = 0; m < count && !rc; m++)
+                for (int c = 0; c < (ctx->visc == 1 ? 1 : dim) && !rc; c++)
+                    for (int par = 0; par < 2 && !rc; par++)
+                        with_dim_wall_visc(dim, ctx->visc, [&](auto D, auto V) {
+                            constexpr int DIM = decltype(D)::value, VISC = decltype(V)::value;
+                            k_stag_gs_w<T, DIM, VISC><<<grd, blk, 0, ctx->stream>>>(
+                                L.g, ctx->walls, A, L.phi[0], L.phi[1], L.phi[2], L.rhs[0], L.rhs[1], L.rhs[2], c, par,
+                                omega);
+                            rc |= post(ctx);
+                        });
+            return rc;
+        }
+        // the colours of the reference's smoother, each as Lphi and the
+        // diagonal of its faces, then the update (the wall faces stay zero)
         for (int m = 0; m < count && !rc; m++)
             for (int color = 1; color <= 2 * dim && !rc; color++)
                 with_dim_wall_visc(dim, ctx->visc, [&](auto D, auto V) {
@@ -833,8 +850,8 @@ static int coarse_first(fhd_ctx* ctx, int n, F bytes) {
 template <typename T>
 static int stag_coarse_first(fhd_ctx* ctx, Multigrid<T>& M) {
     const int dim = ctx->dim;
-    // the single-CTA coarse kernel knows no walls: every level by launches
-    if (ctx->has_walls) return (int)M.s.size();
+    // the single-CTA coarse kernel knows walls for visc_type 1 only
+    if (ctx->has_walls && ctx->visc != 1) return (int)M.s.size();
     return coarse_first(ctx, (int)M.s.size(),
                         [&](int l) { return (size_t)(3 * dim) * (size_t)M.s[l].g.nc * sizeof(T); });
 }
@@ -857,8 +874,9 @@ static int stag_coarse(fhd_ctx* ctx, Multigrid<T>& M, int lc) {
     a.n_down = ctx->p.stag_mg_nsmooths_down;
     a.n_up = ctx->p.stag_mg_nsmooths_up;
     a.n_bottom = ctx->p.stag_mg_nsmooths_bottom;
-    a.jacobi = ctx->p.stag_mg_smoother == 0;
+    a.jacobi = ctx->p.stag_mg_smoother == 0 && !ctx->has_walls;  // (levels with walls smooth by colours)
     a.omega = (T)ctx->p.stag_mg_omega;
+    a.walls = ctx->walls;
     for (int c = 0; c < dim; c++) {
         a.phi[c] = M.s[lc].phi[c];
         a.rhs[c] = M.s[lc].rhs[c];
@@ -873,6 +891,16 @@ static int stag_coarse(fhd_ctx* ctx, Multigrid<T>& M, int lc) {
     }
     const size_t smem = off * sizeof(T);
     int rc = 0;
+    if (ctx->has_walls) {
+        with_dim(dim, [&](auto D) {
+            constexpr int DIM = decltype(D)::value;
+            rc |= rb_allow_smem(k_stag_coarse<T, DIM, 1, true>, smem);
+            if (rc) return;
+            k_stag_coarse<T, DIM, 1, true><<<1, CS_THREADS, smem, ctx->stream>>>(a);
+            rc |= post(ctx);
+        });
+        return rc;
+    }
     with_dim_visc(dim, ctx->visc, [&](auto D, auto V) {
         constexpr int DIM = decltype(D)::value, VISC = decltype(V)::value;
         rc |= rb_allow_smem(k_stag_coarse<T, DIM, VISC>, smem);
