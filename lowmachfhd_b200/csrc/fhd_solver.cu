@@ -13,7 +13,7 @@
 #include <map>
 
 #include "fhd_solver.cuh"
-#include "fhd_coarse.cuh"
+#include "fhd_t2.cuh"
 #include "fhd_rbx.cuh"
 
 namespace fhd {
@@ -156,7 +156,8 @@ static int build_mg(fhd_ctx* ctx, Multigrid<T>& M) {
                 L.alpha[c] = L.own_alpha0[c];
             }
         }
-        L.zm_ok = dim == 3 && stag_zm_pick<T>(L.g, 1, ctx->sms, L.zm[0]) && stag_zm_pick<T>(L.g, 2, ctx->sms, L.zm[1]);
+        L.zm_ok = dim == 2 ? all_even(L.g) && nc < (1ll << 31)
+                           : stag_zm_pick<T>(L.g, 1, ctx->sms, L.zm[0]) && stag_zm_pick<T>(L.g, 2, ctx->sms, L.zm[1]);
     }
     const int ncl = nlevs_mg(ctx->g0, ctx->p.mg_minwidth);
     M.c.resize(ncl);
@@ -651,8 +652,9 @@ static int stag_smooths_planned(fhd_ctx* ctx, StagLevel<T>& L, const SmoothPlan&
     return 0;
 }
 
-// whether a level smooths with the z-march: 3D, even extents of at least
-// four cells, constant viscosity without cross terms; not where a caller
+// whether a level smooths with the z-march (3D, even extents of at least four
+// cells) or on tiles (2D, even extents: fhd_t2.cuh): constant viscosity
+// without cross terms; not where a caller
 // forced or imported a plan, or asked for colour launches (fhd_ctx_set_fused
 // 0).  It is the fastest form at every size it takes (a pair of smooths,
 // FP32, before and now: 40^3 52 -> 9 us, 128^3 64 -> 44, 192^3 238 -> 113,
@@ -682,7 +684,18 @@ static int stag_zm_launch(fhd_ctx* ctx, StagLevel<T>& L, int ns, int zero) {
     }
     const dim3 grd(G.tx * G.ty, G.chunks, 3);
     const T omega = (T)ctx->p.stag_mg_omega;
-    if (ns == 1) {
+    if (ctx->dim == 2) {
+        T2Args<T> Q;
+        for (int c = 0; c < 2; c++) {
+            Q.src[c] = L.phi[c];
+            Q.dst[c] = L.tmp[c];
+            Q.rhs[c] = L.rhs[c];
+        }
+        if (ns == 1)
+            k_stag_t2<T, 1><<<t2_grid(L.g, 1), T2_THREADS, 0, ctx->stream>>>(L.g.n[0], L.g.n[1], L.op(), Q, omega, zero);
+        else
+            k_stag_t2<T, 2><<<t2_grid(L.g, 2), T2_THREADS, 0, ctx->stream>>>(L.g.n[0], L.g.n[1], L.op(), Q, omega, zero);
+    } else if (ns == 1) {
         if (int rc = rb_allow_smem(k_stag_zm<T, 1>, G.smem)) return rc;
         k_stag_zm<T, 1><<<grd, G.threads, G.smem, ctx->stream>>>(L.g, G, L.op(), R, omega, zero);
     } else {
@@ -1180,12 +1193,57 @@ static int cc_rb_pairs(fhd_ctx* ctx, CCLevel<T>& C, const RBGeom& G, int pairs) 
     return 0;
 }
 
+// whether a level smooths on tiles (fhd_t2.cuh): 2D, even extents; not where a
+// caller forced or imported a plan, or asked for colour launches
+// (fhd_ctx_set_fused 0).  One launch in place of four, at every size in use: no
+// plan is timed against it.
 template <typename T>
-static int cc_smooths(fhd_ctx* ctx, CCLevel<T>& C, int count) {
+static bool cc_t2_use(fhd_ctx* ctx, const CCLevel<T>& C) {
+    return ctx->dim == 2 && all_even(C.g) && C.g.nc < (1ll << 31) && ctx->fused_mode != 0 &&
+           (C.plan.kind < 0 || C.plan.march) && rb_aligned(C.phi) && rb_aligned(C.tmp) && rb_aligned(C.rhs) &&
+           rb_aligned(C.a[0]) && rb_aligned(C.a[1]);
+}
+
+// one launch of ns smooths phi -> tmp; the two buffers then change names
+template <typename T>
+static int cc_t2_launch(fhd_ctx* ctx, CCLevel<T>& C, int ns, int zero) {
+    const dim3 grd = t2_grid(C.g, ns);
+    if (ns == 1)
+        k_cc_t2<T, 1><<<grd, T2_THREADS, 0, ctx->stream>>>(C.g.n[0], C.g.n[1], C.op(), C.phi, C.tmp, C.rhs, zero);
+    else
+        k_cc_t2<T, 2><<<grd, T2_THREADS, 0, ctx->stream>>>(C.g.n[0], C.g.n[1], C.op(), C.phi, C.tmp, C.rhs, zero);
+    FHD_POST(ctx);
+    std::swap(C.phi, C.tmp);
+    C.away = !C.away;
+    return 0;
+}
+
+// count smooths of a level.  zero: the unknowns are zero and need not be
+// stored so (tiles only).  home: the last smooths of the level in a V-cycle
+// (see stag_zm_smooths).
+template <typename T>
+static int cc_smooths(fhd_ctx* ctx, CCLevel<T>& C, int count, int zero = 0, bool home = true) {
     int m0 = 0;
     RBGeom G;
     const bool aligned = rb_aligned(C.phi) && rb_aligned(C.tmp) && rb_aligned(C.rhs);
-    if (C.plan.kind >= 0 && aligned && all_even(C.g)) {
+    if (cc_t2_use(ctx, C)) {
+        int pairs = count / 2, ones = count & 1;
+        if (home && (((pairs + ones) & 1) != 0) != C.away && pairs > 0) {
+            pairs--;
+            ones += 2;
+        }
+        for (; pairs > 0; pairs--, zero = 0)
+            if (int rc = cc_t2_launch(ctx, C, 2, zero)) return rc;
+        for (; ones > 0; ones--, zero = 0)
+            if (int rc = cc_t2_launch(ctx, C, 1, zero)) return rc;
+        if (home && C.away) {
+            FHD_CUDA_TRY(cudaMemcpyAsync(C.tmp, C.phi, sizeof(T) * C.g.nc, cudaMemcpyDeviceToDevice, ctx->stream));
+            std::swap(C.phi, C.tmp);
+            C.away = false;
+        }
+        return 0;
+    }
+    if (C.plan.kind >= 0 && !C.plan.march && aligned && all_even(C.g)) {
         const SmoothPlan& P = C.plan;
         if (P.kind == 1) {
             if (int rc = cc_rb_pairs(ctx, C, P.rb, count / 2)) return rc;
@@ -1427,15 +1485,26 @@ static int tune_levels_locked(fhd_ctx* ctx, Multigrid<T>& M, std::vector<T*>& sc
             continue;
         }
         std::vector<SmoothPlan> cands = cc_cands(ctx, C);
+        const int nlist = (int)cands.size();
+        SmoothPlan march;  // the tiles: one past the list
+        march.kind = 1;
+        march.march = true;
+        march.ncand = nlist;
+        march.index = nlist;
+        const bool can_march = cc_t2_use(ctx, C);
         if (force >= 0) {
-            C.plan = cands[(size_t)force < cands.size() ? force : 0];
-            C.plan.ncand = (int)cands.size();
+            if (force == nlist && can_march) {
+                C.plan = march;
+            } else {
+                C.plan = cands[force < nlist ? force : 0];
+                C.plan.ncand = nlist;
+            }
             continue;
         }
         auto im = g_tune_import.find(key);
-        if (im != g_tune_import.end() && im->second < (int)cands.size()) {
-            C.plan = cands[im->second];
-            C.plan.ncand = (int)cands.size();
+        if (im != g_tune_import.end() && (im->second < nlist || (im->second == nlist && can_march))) {
+            C.plan = im->second < nlist ? cands[im->second] : march;
+            C.plan.ncand = nlist;
             C.plan.index = im->second;
             g_tune[key] = C.plan;
             continue;
@@ -1445,6 +1514,14 @@ static int tune_levels_locked(fhd_ctx* ctx, Multigrid<T>& M, std::vector<T*>& sc
         S.phi = scratch[0];
         S.tmp = scratch[1];
         S.rhs = scratch[2];
+        if (can_march) {  // fastest wherever it runs (cc_t2_use): timed for the record only
+            S.plan = march;
+            if (int rc = time_pairs(ctx, ev[0], ev[1], [&]() { return cc_t2_launch(ctx, S, 2, 0); }, march.us))
+                return rc;
+            C.plan = march;
+            g_tune[key] = C.plan;
+            continue;
+        }
         int best = -1;
         for (size_t i = 0; i < cands.size(); i++) {
             float us = 0.f;
@@ -1527,15 +1604,23 @@ static int cc_coarse(fhd_ctx* ctx, Multigrid<T>& M, int lc) {
     return rc;
 }
 
-// V-cycle from level l; levels from lc down run in the coarse kernel
+// whether level l starts its V-cycle from zeros that are not stored
 template <typename T>
-static int cc_vcycle(fhd_ctx* ctx, Multigrid<T>& M, int l, int lc) {
+static bool cc_from_zero(fhd_ctx* ctx, Multigrid<T>& M, int l, int lc) {
+    const int n = l < (int)M.c.size() - 1 ? ctx->p.mg_nsmooths_down : ctx->p.mg_nsmooths_bottom;
+    return l < lc && n > 0 && cc_t2_use(ctx, M.c[l]);
+}
+
+// V-cycle from level l; levels from lc down run in the coarse kernel.  zero:
+// the unknowns of level l start at zero, whatever is stored there
+template <typename T>
+static int cc_vcycle(fhd_ctx* ctx, Multigrid<T>& M, int l, int lc, int zero) {
     const int nl = (int)M.c.size();
     CCLevel<T>& C = M.c[l];
     if (l == lc) return cc_coarse(ctx, M, lc);
-    if (l == nl - 1) return cc_smooths(ctx, C, ctx->p.mg_nsmooths_bottom);
+    if (l == nl - 1) return cc_smooths(ctx, C, ctx->p.mg_nsmooths_bottom, zero);
     {
-        int rc = cc_smooths(ctx, C, ctx->p.mg_nsmooths_down);
+        int rc = cc_smooths(ctx, C, ctx->p.mg_nsmooths_down, zero, false);
         if (rc) return rc;
     }
     CCLevel<T>& D = M.c[l + 1];
@@ -1547,8 +1632,9 @@ static int cc_vcycle(fhd_ctx* ctx, Multigrid<T>& M, int l, int lc) {
         rc |= post(ctx);
     });
     if (rc) return rc;
-    if (l + 1 != lc) FHD_CUDA_TRY(cudaMemsetAsync(D.phi, 0, sizeof(T) * D.g.nc, ctx->stream));
-    rc = cc_vcycle(ctx, M, l + 1, lc);
+    const bool zero_d = cc_from_zero(ctx, M, l + 1, lc);
+    if (l + 1 != lc && !zero_d) FHD_CUDA_TRY(cudaMemsetAsync(D.phi, 0, sizeof(T) * D.g.nc, ctx->stream));
+    rc = cc_vcycle(ctx, M, l + 1, lc, zero_d);
     if (rc) return rc;
     with_dim(ctx->dim, [&](auto Dm) {
         constexpr int DIM = decltype(Dm)::value;
@@ -1561,11 +1647,13 @@ static int cc_vcycle(fhd_ctx* ctx, Multigrid<T>& M, int l, int lc) {
 
 // Phi = 0, then mg_max_vcycles V-cycles on M.c[0].rhs
 template <typename T>
-static int cc_solve(fhd_ctx* ctx, Multigrid<T>& M) {
+static int cc_cycles(fhd_ctx* ctx, Multigrid<T>& M) {
     CCLevel<T>& C = M.c[0];
     const i64 nc = C.g.nc;
-    FHD_CUDA_TRY(cudaMemsetAsync(C.phi, 0, sizeof(T) * nc, ctx->stream));
     const int maxv = ctx->p.mg_max_vcycles;
+    const int lc = cc_coarse_first(ctx, M);
+    const bool zero = maxv == 1 && cc_from_zero(ctx, M, 0, lc);
+    if (!zero) FHD_CUDA_TRY(cudaMemsetAsync(C.phi, 0, sizeof(T) * nc, ctx->stream));
     double r0 = 1.0;
     if (maxv > 1) {
         k_maxabs<T><<<flat_blocks(nc), RED_THREADS, 0, ctx->stream>>>(nc, C.rhs, slot(ctx, S_MG));
@@ -1575,9 +1663,8 @@ static int cc_solve(fhd_ctx* ctx, Multigrid<T>& M) {
         r0 = ctx->hscal[S_MG];
         if (r0 == 0.0) return 0;
     }
-    const int lc = cc_coarse_first(ctx, M);
     for (int vc = 1; vc <= maxv; vc++) {
-        int rc = cc_vcycle(ctx, M, 0, lc);
+        int rc = cc_vcycle(ctx, M, 0, lc, zero);
         if (rc) return rc;
         if (vc == maxv) break;
         with_dim(ctx->dim, [&](auto D) {
@@ -1594,6 +1681,19 @@ static int cc_solve(fhd_ctx* ctx, Multigrid<T>& M) {
     }
     ctx->vcycles += maxv;
     return 0;
+}
+
+// the pressure solve; on an error the levels' buffers get their names back
+template <typename T>
+static int cc_solve(fhd_ctx* ctx, Multigrid<T>& M) {
+    const int rc = cc_cycles(ctx, M);
+    if (rc)
+        for (auto& C : M.c)
+            if (C.away) {
+                std::swap(C.phi, C.tmp);
+                C.away = false;
+            }
+    return rc;
 }
 
 // ---------------------------------------------------------------------

@@ -205,6 +205,7 @@ struct CCLevel {
     T* phi = nullptr;
     T* rhs = nullptr;
     T* tmp = nullptr;
+    bool away = false;  // phi and tmp are exchanged
     CCOp<T> op() const {
         CCOp<T> A;
         for (int c = 0; c < 3; c++) A.a[c] = a[c];
