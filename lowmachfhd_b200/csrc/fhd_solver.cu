@@ -727,7 +727,7 @@ static int stag_zm_smooths(fhd_ctx* ctx, StagLevel<T>& L, int count, int zero, b
     for (; ones > 0; ones--, zero = 0)
         if (int rc = stag_zm_launch(ctx, L, 1, zero)) return rc;
     if (home && L.away) {
-        for (int c = 0; c < 3; c++) {
+        for (int c = 0; c < ctx->dim; c++) {
             FHD_CUDA_TRY(cudaMemcpyAsync(L.tmp[c], L.phi[c], sizeof(T) * L.g.nc, cudaMemcpyDeviceToDevice, ctx->stream));
             std::swap(L.phi[c], L.tmp[c]);
         }
