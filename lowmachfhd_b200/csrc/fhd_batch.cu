@@ -32,7 +32,7 @@
 #include <vector>
 
 #include "fhd_solver.cuh"
-#include "fhd_coarse.cuh"
+#include "fhd_t2.cuh"
 #include "fhd_vec.cuh"
 
 namespace fhd {
@@ -143,28 +143,41 @@ __device__ __forceinline__ CCOp<T> box_ccop(const T* ones, double dx) {
 // ---------------------------------------------------------------------
 // staggered multigrid, per-level launches over (box, tile) tables
 // ---------------------------------------------------------------------
-// one colour of the 4-colour Gauss-Seidel (k_stag_gs): component C, faces
-// with (i+j) % 2 == par
-template <typename T, int C>
-__global__ void __launch_bounds__(256) kb_stag_gs(const Tile* tiles, int n, const Lev* lev, int l, const Ctl* ctl, int mode,
-                                                  T* const* phi, const T* const* rhs, const T* ones, T theta,
-                                                  int par, T omega) {
+// NS red-black smooths of both components, src -> dst (fhd_t2.cuh); tiles of
+// t2_tx x t2_ty cells
+template <typename T, int NS>
+__global__ void __launch_bounds__(256) kb_stag_t2(const Tile* tiles, int n, const Lev* lev, int l, const Ctl* ctl, int mode,
+                                                  T* const* src, T* const* dst, const T* const* rhs, const T* ones,
+                                                  T theta, T omega, int zero) {
+    __shared__ T sm[4 * 32 * T2_EY];
+    for_tiles(tiles, n, ctl, mode, [&](const Tile& t, int q) {
+        const Lev L = lev[t.box * MAXL + l];
+        CSVisc1<T, 2> U;
+        U.set(box_op<T>(ones, theta, ctl[t.box].eta, L.g.dx), omega);
+        const T* const sp[2] = {src[0] + L.off, src[1] + L.off};
+        T* const dp[2] = {dst[0] + L.off, dst[1] + L.off};
+        const T* const rp[2] = {rhs[0] + L.off, rhs[1] + L.off};
+        const T* const al[2] = {ones, ones};
+        __syncthreads();  // the last tile's shared memory
+        t2_stag<T, NS, true>(L.g.n[0], L.g.n[1], t.i0, t.j0, sp, dp, rp, al, U, zero, (L.off & 1) == 0, sm);
+    });
+}
+
+// src -> dst on the tiles of the covered boxes (a level that ends its smooths
+// in the second buffer; boxes that solve it in their coarse kernel keep theirs)
+template <typename T>
+__global__ void __launch_bounds__(256) kb_copy(const Tile* tiles, int n, const Lev* lev, int l, const Ctl* ctl, int mode,
+                                               const T* src, T* dst) {
     for_tiles(tiles, n, ctl, mode, [&](const Tile& t, int q) {
         const Lev L = lev[t.box * MAXL + l];
         const int j = t.j0 + threadIdx.y;
-        const int i = t.i0 + 2 * threadIdx.x + ((j + par) & 1);
-        if (j >= L.g.n[1] || i >= L.g.n[0]) return;
-        CellF P;
-        P.set(L.g, i, j, 0);
-        T* p0 = phi[0] + L.off;
-        T* p1 = phi[1] + L.off;
-        const T* ph[3] = {p0, p1, nullptr};
-        T* pc = C == 0 ? p0 : p1;
-        const StagOp<T> A = box_op<T>(ones, theta, ctl[t.box].eta, L.g.dx);
-        const i64 f = P.id(0, 0, 0);
-        T dg;
-        const T Lv = stag_lface<T, 2, 1, C>(A, ph, P, dg);
-        pc[f] = pc[f] + sm_quot(omega * (ld(rhs[C] + L.off, f) - Lv), dg);
+        if (j >= L.g.n[1]) return;
+    #pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int i = t.i0 + threadIdx.x + 32 * u;
+            const i64 f = L.off + (i64)i + (i64)L.g.n[0] * j;
+            if (i < L.g.n[0]) dst[f] = src[f];
+        }
     });
 }
 
@@ -224,11 +237,10 @@ __global__ void __launch_bounds__(256) kb_stag_restrict(const Tile* tiles, int n
 }
 
 // stag_prolongation: fine phi (level l) += P coarse phi (level l+1); thread
-// per fine face, the tiles are level l's; phi is the per-level table from
-// level l on (phi[c] level l, phi[2 + c] level l+1)
+// per fine face, the tiles are level l's
 template <typename T>
 __global__ void __launch_bounds__(256) kb_stag_prolong(const Tile* tiles, int n, const Lev* lev, int l, const Ctl* ctl,
-                                                       int mode, T* const* phi) {
+                                                       int mode, T* const* phi, T* const* cphi) {
     for_tiles(tiles, n, ctl, mode, [&](const Tile& t, int q) {
         const Lev F = lev[t.box * MAXL + l], Q = lev[t.box * MAXL + l + 1];
         const int j = t.j0 + threadIdx.y;
@@ -244,7 +256,7 @@ __global__ void __launch_bounds__(256) kb_stag_prolong(const Tile* tiles, int n,
             const i64 f = (i64)i + (i64)F.g.n[0] * j;
     #pragma unroll
             for (int c = 0; c < 2; c++) {
-                const T* Cp = phi[2 + c] + Q.off;
+                const T* Cp = cphi[c] + Q.off;
                 const int ca = (c == 0) ? 1 : 0;
                 const int oa = (I[ca] & 1) ? 1 : -1;
                 const T v = stag_prolong_expr<T, 2>((I[c] & 1) == 0, oa, 0, [&](int o, int pa, int pb) {
@@ -269,22 +281,16 @@ __global__ void __launch_bounds__(CS_THREADS) kb_stag_coarse(const StagCoarseArg
 // ---------------------------------------------------------------------
 // pressure multigrid
 // ---------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(256) kb_cc_gsrb(const Tile* tiles, int n, const Lev* lev, int l, const Ctl* ctl, int mode,
-                                                  T* phi, const T* rhs, const T* ones, int par) {
+// NS red-black smooths, src -> dst (fhd_t2.cuh)
+template <typename T, int NS>
+__global__ void __launch_bounds__(256) kb_cc_t2(const Tile* tiles, int n, const Lev* lev, int l, const Ctl* ctl, int mode,
+                                                const T* src, T* dst, const T* rhs, int zero) {
+    __shared__ T sm[2 * 32 * T2_EY];
     for_tiles(tiles, n, ctl, mode, [&](const Tile& t, int q) {
         const Lev L = lev[t.box * MAXL + l];
-        const int j = t.j0 + threadIdx.y;
-        const int i = t.i0 + 2 * threadIdx.x + ((j + par) & 1);
-        if (j >= L.g.n[1] || i >= L.g.n[0]) return;
-        CellF P;
-        P.set(L.g, i, j, 0);
-        const CCOp<T> A = box_ccop<T>(ones, L.g.dx);
-        T* ph = phi + L.off;
-        T dg;
-        const T Lv = cc_lap<T, 2>(A, ph, P, dg);
-        const i64 f = P.id(0, 0, 0);
-        ph[f] = ph[f] + sm_quot(ld(rhs + L.off, f) - Lv, dg);
+        __syncthreads();  // the last tile's shared memory
+        t2_cc<T, NS, true>(L.g.n[0], L.g.n[1], t.i0, t.j0, src + L.off, dst + L.off, rhs + L.off, nullptr, nullptr,
+                           T(1.0 / (L.g.dx * L.g.dx)), zero, (L.off & 1) == 0, sm);
     });
 }
 
@@ -990,6 +996,9 @@ struct fhd_batch {
     // per-level launch tables: boxes whose level l is above their coarse end
     std::vector<Tile*> tab_s, tab_c;
     std::vector<int> ntab_s, ntab_c;
+    // the same for the smoothers' tiles, with one and two smooths per launch
+    std::vector<Tile*> t2_s[2], t2_c[2];
+    std::vector<int> nt2_s[2], nt2_c[2];
     // restriction targets: level l of the boxes that reach it by launches
     // (l <= their coarse end), so that the coarse kernel's first level is
     // included
@@ -1070,9 +1079,9 @@ Grid grid2(int nx, int ny, double dx) {
     return g;
 }
 
-void tiles_of(std::vector<Tile>& v, int box, int nx, int ny) {
-    for (int j0 = 0; j0 < ny; j0 += TY)
-        for (int i0 = 0; i0 < nx; i0 += TX) v.push_back(Tile{box, i0, j0});
+void tiles_of(std::vector<Tile>& v, int box, int nx, int ny, int tx = TX, int ty = TY) {
+    for (int j0 = 0; j0 < ny; j0 += ty)
+        for (int i0 = 0; i0 < nx; i0 += tx) v.push_back(Tile{box, i0, j0});
 }
 
 template <typename T>
@@ -1157,6 +1166,15 @@ int build(fhd_batch* B) {
         }
         B->ntab_s[l] = (int)v.size();
         B->tab_s[l] = upload_tiles(v);
+        for (int ns = 1; ns <= 2; ns++) {
+            std::vector<Tile> w;
+            for (int b = 0; b < nb; b++)
+                if (l < B->lcs[b])
+                    tiles_of(w, b, ls[(size_t)b * MAXL + l].g.n[0], ls[(size_t)b * MAXL + l].g.n[1], t2_tx(ns),
+                             t2_ty(ns));
+            B->nt2_s[ns - 1].push_back((int)w.size());
+            B->t2_s[ns - 1].push_back(upload_tiles(w));
+        }
         B->nall_s[l] = (int)a.size();
         B->all_s[l] = upload_tiles(a);
     }
@@ -1174,6 +1192,15 @@ int build(fhd_batch* B) {
         }
         B->ntab_c[l] = (int)v.size();
         B->tab_c[l] = upload_tiles(v);
+        for (int ns = 1; ns <= 2; ns++) {
+            std::vector<Tile> w;
+            for (int b = 0; b < nb; b++)
+                if (l < B->lcc[b])
+                    tiles_of(w, b, lc[(size_t)b * MAXL + l].g.n[0], lc[(size_t)b * MAXL + l].g.n[1], t2_tx(ns),
+                             t2_ty(ns));
+            B->nt2_c[ns - 1].push_back((int)w.size());
+            B->t2_c[ns - 1].push_back(upload_tiles(w));
+        }
         B->nall_c[l] = (int)a.size();
         B->all_c[l] = upload_tiles(a);
     }
@@ -1243,7 +1270,7 @@ int build(fhd_batch* B) {
         memset(&a, 0, sizeof(a));
         const int l0 = B->lcs[b];
         a.nlev = B->nls[b] - l0;
-        a.load_phi = l0 == 0;
+        a.load_phi = 0;  // every V-cycle starts from zero
         a.n_down = B->p.stag_mg_nsmooths_down;
         a.n_up = B->p.stag_mg_nsmooths_up;
         a.n_bottom = B->p.stag_mg_nsmooths_bottom;
@@ -1276,7 +1303,7 @@ int build(fhd_batch* B) {
         memset(&cq, 0, sizeof(cq));
         const int m0 = B->lcc[b];
         cq.nlev = B->nlc[b] - m0;
-        cq.load_phi = m0 == 0;
+        cq.load_phi = 0;
         cq.n_down = B->p.mg_nsmooths_down;
         cq.n_up = B->p.mg_nsmooths_up;
         cq.n_bottom = B->p.mg_nsmooths_bottom;
@@ -1385,23 +1412,51 @@ int seg(fhd_batch* B, int mode, int which, int ncomp = 1) {
     return 0;
 }
 
+// count smooths as launches of two and of one, each from one buffer of the
+// level into the other.  away: whether the unknowns are in the second buffer
+// (in and out).  home: they shall end in the first, so that when the launches
+// would not leave them there the last pair goes as two.
+struct SmoothRuns {
+    int pairs, ones;
+    SmoothRuns(int count, bool away, bool home) : pairs(count / 2), ones(count & 1) {
+        if (home && (((pairs + ones) & 1) != 0) != away && pairs > 0) {
+            pairs--;
+            ones += 2;
+        }
+    }
+};
+
 template <typename T>
-int stag_smooth(fhd_batch* B, int l, int mode, T theta, int count) {
+int stag_smooth(fhd_batch* B, int l, int mode, T theta, int count, int zero, bool& away, bool home) {
     if (!B->ntab_s[l]) return 0;
-    T* const* phi = (T* const*)(B->dsphi + 2 * l);
+    void** buf[2] = {B->dsphi + 2 * l, B->dstmp + 2 * l};
     const T* const* rhs = (const T* const*)(B->dsrhs + 2 * l);
     const T omega = (T)B->p.stag_mg_omega;
-    for (int s = 0; s < count; s++)
-        for (int color = 1; color <= 4; color++) {
-            const int par = (color + 1) & 1;
-            if (color <= 2)
-                kb_stag_gs<T, 0><<<tgrid(B, kb_stag_gs<T, 0>, B->ntab_s[l]), TB, 0, B->stream>>>(B->tab_s[l], B->ntab_s[l], B->dlev_s, l, B->ctl, mode, phi,
-                                                                    rhs, (const T*)B->ones, theta, par, omega);
-            else
-                kb_stag_gs<T, 1><<<tgrid(B, kb_stag_gs<T, 1>, B->ntab_s[l]), TB, 0, B->stream>>>(B->tab_s[l], B->ntab_s[l], B->dlev_s, l, B->ctl, mode, phi,
-                                                                    rhs, (const T*)B->ones, theta, par, omega);
+    const SmoothRuns R(count, away, home);
+    for (int q = 0; q < R.pairs + R.ones; q++) {
+        T* const* src = (T* const*)buf[away];
+        T* const* dst = (T* const*)buf[!away];
+        if (q < R.pairs)
+            kb_stag_t2<T, 2><<<tgrid(B, kb_stag_t2<T, 2>, B->nt2_s[1][l]), TB, 0, B->stream>>>(
+                B->t2_s[1][l], B->nt2_s[1][l], B->dlev_s, l, B->ctl, mode, src, dst, rhs, (const T*)B->ones, theta, omega,
+                zero);
+        else
+            kb_stag_t2<T, 1><<<tgrid(B, kb_stag_t2<T, 1>, B->nt2_s[0][l]), TB, 0, B->stream>>>(
+                B->t2_s[0][l], B->nt2_s[0][l], B->dlev_s, l, B->ctl, mode, src, dst, rhs, (const T*)B->ones, theta, omega,
+                zero);
+        BPOST(B);
+        away = !away;
+        zero = 0;
+    }
+    if (home && away) {
+        for (int c = 0; c < 2; c++) {
+            kb_copy<T><<<tgrid(B, kb_copy<T>, B->ntab_s[l]), TB, 0, B->stream>>>(
+                B->tab_s[l], B->ntab_s[l], B->dlev_s, l, B->ctl, mode, (const T*)B->stmp[2 * l + c],
+                (T*)B->sphi[2 * l + c]);
             BPOST(B);
         }
+        away = false;
+    }
     return 0;
 }
 
@@ -1410,22 +1465,32 @@ int stag_smooth(fhd_batch* B, int l, int mode, T theta, int count) {
 template <typename T>
 int stag_vcycle(fhd_batch* B, int mode, T theta) {
     cudaStream_t st = B->stream;
-    for (int l = 1; l < B->Ls; l++)
-        for (int c = 0; c < 2; c++)
-            if (cudaMemsetAsync(B->sphi[2 * l + c], 0, sizeof(T) * B->Ns[l], st) != cudaSuccess) return FHD_ERR_CUDA;
+    std::vector<char> away(B->Ls, 0);  // level's unknowns in its second buffer
+    auto smooth = [&](int l, int count, int zero, bool home) {
+        bool w = away[l] != 0;
+        const int rc = stag_smooth<T>(B, l, mode, theta, count, zero, w, home);
+        away[l] = w;
+        return rc;
+    };
+    const int nd = B->p.stag_mg_nsmooths_down, nu = B->p.stag_mg_nsmooths_up;
     for (int l = 0; l + 1 < B->Ls; l++) {
         if (!B->ntab_s[l]) continue;
-        int rc = stag_smooth<T>(B, l, mode, theta, B->p.stag_mg_nsmooths_down);
+        // (with no smooth on the way down the zeros are stored)
+        for (int c = 0; c < 2 && nd < 1; c++)
+            if (cudaMemsetAsync(B->sphi[2 * l + c], 0, sizeof(T) * B->Ns[l], st) != cudaSuccess) return FHD_ERR_CUDA;
+        int rc = smooth(l, nd, 1, false);
         if (rc) return rc;
-        kb_stag_resid<T><<<tgrid(B, kb_stag_resid<T>, B->ntab_s[l]), TB, 0, st>>>(B->tab_s[l], B->ntab_s[l], B->dlev_s, l, B->ctl, mode,
-                                                       (T* const*)(B->dsphi + 2 * l), (const T* const*)(B->dsrhs + 2 * l),
-                                                       (T* const*)(B->dstmp + 2 * l), (const T*)B->ones, theta);
+        void** phi = away[l] ? B->dstmp + 2 * l : B->dsphi + 2 * l;
+        void** tmp = away[l] ? B->dsphi + 2 * l : B->dstmp + 2 * l;
+        kb_stag_resid<T><<<tgrid(B, kb_stag_resid<T>, B->ntab_s[l]), TB, 0, st>>>(
+            B->tab_s[l], B->ntab_s[l], B->dlev_s, l, B->ctl, mode, (T* const*)phi, (const T* const*)(B->dsrhs + 2 * l),
+            (T* const*)tmp, (const T*)B->ones, theta);
         BPOST(B);
         // the restriction's targets: level l+1 of the boxes smoothing level l
         // by launches (it may be their coarse kernel's first level)
-        kb_stag_restrict<T><<<tgrid(B, kb_stag_restrict<T>, B->nall_s[l + 1]), TB, 0, st>>>(B->all_s[l + 1], B->nall_s[l + 1], B->dlev_s, l, B->ctl, mode,
-                                                            (T* const*)(B->dstmp + 2 * l),
-                                                            (T* const*)(B->dsrhs + 2 * (l + 1)));
+        kb_stag_restrict<T><<<tgrid(B, kb_stag_restrict<T>, B->nall_s[l + 1]), TB, 0, st>>>(
+            B->all_s[l + 1], B->nall_s[l + 1], B->dlev_s, l, B->ctl, mode, (T* const*)tmp,
+            (T* const*)(B->dsrhs + 2 * (l + 1)));
         BPOST(B);
     }
     kb_stag_coarse<T><<<B->nbox, CS_THREADS, B->smem_s, st>>>((const StagCoarseArgs<T>*)B->sargs, B->ord_s, B->ctl,
@@ -1433,37 +1498,55 @@ int stag_vcycle(fhd_batch* B, int mode, T theta) {
     BPOST(B);
     for (int l = B->Ls - 2; l >= 0; l--) {
         if (!B->ntab_s[l]) continue;
-        kb_stag_prolong<T><<<tgrid(B, kb_stag_prolong<T>, B->ntab_s[l]), TB, 0, st>>>(B->tab_s[l], B->ntab_s[l], B->dlev_s, l, B->ctl, mode,
-                                                         (T* const*)(B->dsphi + 2 * l));
+        kb_stag_prolong<T><<<tgrid(B, kb_stag_prolong<T>, B->ntab_s[l]), TB, 0, st>>>(
+            B->tab_s[l], B->ntab_s[l], B->dlev_s, l, B->ctl, mode,
+            (T* const*)(away[l] ? B->dstmp + 2 * l : B->dsphi + 2 * l), (T* const*)(B->dsphi + 2 * (l + 1)));
         BPOST(B);
-        int rc = stag_smooth<T>(B, l, mode, theta, B->p.stag_mg_nsmooths_up);
+        int rc = smooth(l, nu, 0, true);
         if (rc) return rc;
     }
     return 0;
 }
 
-// Phi = 0, one pressure V-cycle of every covered box on cc level 0's rhs
+// one pressure V-cycle from Phi = 0 of every covered box on cc level 0's rhs
 template <typename T>
 int cc_vcycle(fhd_batch* B, int mode) {
     cudaStream_t st = B->stream;
-    for (int l = 0; l < B->Lc; l++)
-        if (cudaMemsetAsync(B->cphi[l], 0, sizeof(T) * B->Nc[l], st) != cudaSuccess) return FHD_ERR_CUDA;
-    auto smooth = [&](int l, int count) -> int {
-        for (int s = 0; s < count; s++)
-            for (int par = 0; par < 2; par++) {
-                kb_cc_gsrb<T><<<tgrid(B, kb_cc_gsrb<T>, B->ntab_c[l]), TB, 0, st>>>(B->tab_c[l], B->ntab_c[l], B->dlev_c, l, B->ctl, mode, (T*)B->cphi[l],
-                                                          (const T*)B->crhs[l], (const T*)B->ones, par);
-                BPOST(B);
-            }
+    std::vector<char> away(B->Lc, 0);
+    auto smooth = [&](int l, int count, int zero, bool home) -> int {
+        T* buf[2] = {(T*)B->cphi[l], (T*)B->ctmp[l]};
+        const SmoothRuns R(count, away[l] != 0, home);
+        for (int q = 0; q < R.pairs + R.ones; q++) {
+            const T* src = buf[away[l] ? 1 : 0];
+            T* dst = buf[away[l] ? 0 : 1];
+            if (q < R.pairs)
+                kb_cc_t2<T, 2><<<tgrid(B, kb_cc_t2<T, 2>, B->nt2_c[1][l]), TB, 0, st>>>(
+                    B->t2_c[1][l], B->nt2_c[1][l], B->dlev_c, l, B->ctl, mode, src, dst, (const T*)B->crhs[l], zero);
+            else
+                kb_cc_t2<T, 1><<<tgrid(B, kb_cc_t2<T, 1>, B->nt2_c[0][l]), TB, 0, st>>>(
+                    B->t2_c[0][l], B->nt2_c[0][l], B->dlev_c, l, B->ctl, mode, src, dst, (const T*)B->crhs[l], zero);
+            BPOST(B);
+            away[l] = !away[l];
+            zero = 0;
+        }
+        if (home && away[l]) {
+            kb_copy<T><<<tgrid(B, kb_copy<T>, B->ntab_c[l]), TB, 0, st>>>(B->tab_c[l], B->ntab_c[l], B->dlev_c, l, B->ctl,
+                                                                        mode, buf[1], buf[0]);
+            BPOST(B);
+            away[l] = 0;
+        }
         return 0;
     };
+    auto phi = [&](int l) { return (T*)(away[l] ? B->ctmp[l] : B->cphi[l]); };
+    const int nd = B->p.mg_nsmooths_down, nu = B->p.mg_nsmooths_up;
     for (int l = 0; l + 1 < B->Lc; l++) {
         if (!B->ntab_c[l]) continue;
-        int rc = smooth(l, B->p.mg_nsmooths_down);
+        if (nd < 1 && cudaMemsetAsync(B->cphi[l], 0, sizeof(T) * B->Nc[l], st) != cudaSuccess) return FHD_ERR_CUDA;
+        int rc = smooth(l, nd, 1, false);
         if (rc) return rc;
-        kb_cc_resid_restrict<T><<<tgrid(B, kb_cc_resid_restrict<T>, B->nall_c[l + 1]), TB, 0, st>>>(B->all_c[l + 1], B->nall_c[l + 1], B->dlev_c, l, B->ctl, mode,
-                                                                (const T*)B->cphi[l], (const T*)B->crhs[l],
-                                                                (T*)B->crhs[l + 1], (const T*)B->ones);
+        kb_cc_resid_restrict<T><<<tgrid(B, kb_cc_resid_restrict<T>, B->nall_c[l + 1]), TB, 0, st>>>(
+            B->all_c[l + 1], B->nall_c[l + 1], B->dlev_c, l, B->ctl, mode, phi(l), (const T*)B->crhs[l],
+            (T*)B->crhs[l + 1], (const T*)B->ones);
         BPOST(B);
     }
     kb_cc_coarse<T><<<B->nbox, CS_THREADS, B->smem_c, st>>>((const CCCoarseArgs<T>*)B->cargs, B->ord_c, B->ctl,
@@ -1471,10 +1554,10 @@ int cc_vcycle(fhd_batch* B, int mode) {
     BPOST(B);
     for (int l = B->Lc - 2; l >= 0; l--) {
         if (!B->ntab_c[l]) continue;
-        kb_cc_prolong<T><<<tgrid(B, kb_cc_prolong<T>, B->ntab_c[l]), TB, 0, st>>>(B->tab_c[l], B->ntab_c[l], B->dlev_c, l, B->ctl, mode, (T*)B->cphi[l],
-                                                      (const T*)B->cphi[l + 1]);
+        kb_cc_prolong<T><<<tgrid(B, kb_cc_prolong<T>, B->ntab_c[l]), TB, 0, st>>>(
+            B->tab_c[l], B->ntab_c[l], B->dlev_c, l, B->ctl, mode, phi(l), (const T*)B->cphi[l + 1]);
         BPOST(B);
-        int rc = smooth(l, B->p.mg_nsmooths_up);
+        int rc = smooth(l, nu, 0, true);
         if (rc) return rc;
     }
     return 0;
@@ -1484,9 +1567,7 @@ int cc_vcycle(fhd_batch* B, int mode) {
 template <typename T>
 int precon(fhd_batch* B, int bv, int xv, int mode, double theta) {
     cudaStream_t st = B->stream;
-    // level-0 velocity unknowns start at zero, rhs = b_u
-    for (int c = 0; c < 2; c++)
-        if (cudaMemsetAsync(B->sphi[c], 0, sizeof(T) * B->N0, st) != cudaSuccess) return FHD_ERR_CUDA;
+    // rhs = b_u (the V-cycle starts from zero)
     kb_to_T<T><<<tgrid(B, kb_to_T<T>, B->ntab0), TB, 0, st>>>(B->tab0, B->ntab0, B->dlev_s, B->ctl, mode, vp(B, bv), (T* const*)B->dsrhs);
     BPOST(B);
     int rc = stag_vcycle<T>(B, mode, (T)theta);

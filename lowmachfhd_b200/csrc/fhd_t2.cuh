@@ -26,13 +26,32 @@ constexpr int T2_THREADS = 32 * T2_WARPS;
 __host__ __device__ constexpr int t2_tx(int ns) { return 64 - 4 * ns; }
 __host__ __device__ constexpr int t2_ty(int ns) { return T2_EY - 4 * ns; }
 
+// a pair of values, as one access where vec says that it is aligned
+template <typename T>
+__device__ __forceinline__ typename Pair2<T>::V t2_ld(const T* p, bool vec) {
+    typedef typename Pair2<T>::V V2;
+    if (vec) return *reinterpret_cast<const V2*>(p);
+    V2 v = {p[0], p[1]};
+    return v;
+}
+template <typename T>
+__device__ __forceinline__ void t2_st(T* p, typename Pair2<T>::V v, bool vec) {
+    if (vec) {
+        *reinterpret_cast<typename Pair2<T>::V*>(p) = v;
+    } else {
+        p[0] = v.x;
+        p[1] = v.y;
+    }
+}
+
 // the thread's place in the tile at (x0, y0) of an nx x ny level (both even)
 struct T2Place {
     int lane, row, e[T2_ROWS];      // e: linear index of its pair's first cell in each row
     bool inner[T2_ROWS], odd[T2_ROWS];  // stored here; red cell at odd x
     __device__ __forceinline__ void set(int nx, int ny, int x0, int y0, int H) {
-        lane = threadIdx.x & 31;
-        row = threadIdx.x >> 5;
+        const int tid = threadIdx.x + blockDim.x * threadIdx.y;
+        lane = tid & 31;
+        row = tid >> 5;
         const int np = nx >> 1, h = (x0 - H) / 2 + lane;  // (x0 and H even; may be negative: exact division)
         int hw = h % np;
         hw = hw < 0 ? hw + np : hw;
@@ -56,11 +75,12 @@ struct T2Place {
     }
 };
 
-// NS smooths of both components of the visc_type 1 operator; sm: 4 x T2_EY x 32
-template <typename T, int NS>
+// NS smooths of both components of the visc_type 1 operator (ONE: alpha = 1);
+// vec: every array is aligned to pairs; sm: 4 x T2_EY x 32
+template <typename T, int NS, bool ONE>
 __device__ __forceinline__ void t2_stag(int nx, int ny, int x0, int y0, const T* const (&src)[2], T* const (&dst)[2],
                                         const T* const (&rhs)[2], const T* const (&alpha)[2],
-                                        const CSVisc1<T, 2>& U, int zero, T* sm) {
+                                        const CSVisc1<T, 2>& U, int zero, bool vec, T* sm) {
     typedef typename Pair2<T>::V V2;
     constexpr int H = 2 * NS, PL = 32 * T2_EY;
     T2Place P;
@@ -72,9 +92,10 @@ __device__ __forceinline__ void t2_stag(int nx, int ny, int x0, int y0, const T*
 #pragma unroll
         for (int c = 0; c < 2; c++) {
             V2 u = {T(0), T(0)};
-            if (!zero) u = *reinterpret_cast<const V2*>(src[c] + P.e[r]);
-            const V2 b = *reinterpret_cast<const V2*>(rhs[c] + P.e[r]);
-            const V2 a = *reinterpret_cast<const V2*>(alpha[c] + P.e[r]);
+            if (!zero) u = t2_ld(src[c] + P.e[r], vec);
+            const V2 b = t2_ld(rhs[c] + P.e[r], vec);
+            V2 a = {T(1), T(1)};
+            if (!ONE) a = t2_ld(alpha[c] + P.e[r], vec);
             const T d0 = U.as * a.x + U.bd, d1 = U.as * a.y + U.bd;
             const bool o = P.odd[r];
             v[0][c][r] = o ? u.y : u.x; v[1][c][r] = o ? u.x : u.y;
@@ -109,14 +130,14 @@ __device__ __forceinline__ void t2_stag(int nx, int ny, int x0, int y0, const T*
                 V2 o;
                 o.x = P.odd[r] ? v[1][c][r] : v[0][c][r];
                 o.y = P.odd[r] ? v[0][c][r] : v[1][c][r];
-                *reinterpret_cast<V2*>(dst[c] + P.e[r]) = o;
+                t2_st(dst[c] + P.e[r], o, vec);
             }
 }
 
 // NS smooths of the pressure operator D a G (ONE: a = 1); sm: 2 x T2_EY x 32
 template <typename T, int NS, bool ONE>
 __device__ __forceinline__ void t2_cc(int nx, int ny, int x0, int y0, const T* src, T* dst, const T* rhs, const T* ax,
-                                      const T* ay, T q, int zero, T* sm) {
+                                      const T* ay, T q, int zero, bool vec, T* sm) {
     typedef typename Pair2<T>::V V2;
     constexpr int H = 2 * NS, PL = 32 * T2_EY;
     T2Place P;
@@ -128,13 +149,12 @@ __device__ __forceinline__ void t2_cc(int nx, int ny, int x0, int y0, const T* s
 #pragma unroll
     for (int r = 0; r < T2_ROWS; r++) {
         V2 u = {T(0), T(0)};
-        if (!zero) u = *reinterpret_cast<const V2*>(src + P.e[r]);
-        const V2 b = *reinterpret_cast<const V2*>(rhs + P.e[r]);
+        if (!zero) u = t2_ld(src + P.e[r], vec);
+        const V2 b = t2_ld(rhs + P.e[r], vec);
         if (!ONE) {
             const int i0 = P.e[r] % nx, row0 = P.e[r] - i0;
             const int en = i0 + 2 == nx ? row0 : P.e[r] + 2, eu = row0 + nx == nx * ny ? i0 : P.e[r] + nx;
-            const V2 a = *reinterpret_cast<const V2*>(ax + P.e[r]);
-            const V2 l = *reinterpret_cast<const V2*>(ay + P.e[r]), h = *reinterpret_cast<const V2*>(ay + eu);
+            const V2 a = t2_ld(ax + P.e[r], vec), l = t2_ld(ay + P.e[r], vec), h = t2_ld(ay + eu, vec);
             cx[0][r] = a.x; cx[1][r] = a.y; cx[2][r] = ax[en];
             cl[0][r] = l.x; cl[1][r] = l.y; ch[0][r] = h.x; ch[1][r] = h.y;
         }
@@ -177,7 +197,7 @@ __device__ __forceinline__ void t2_cc(int nx, int ny, int x0, int y0, const T* s
             V2 o;
             o.x = P.odd[r] ? v[1][r] : v[0][r];
             o.y = P.odd[r] ? v[0][r] : v[1][r];
-            *reinterpret_cast<V2*>(dst + P.e[r]) = o;
+            t2_st(dst + P.e[r], o, vec);
         }
 }
 
@@ -194,7 +214,7 @@ __global__ void __launch_bounds__(T2_THREADS) k_stag_t2(int nx, int ny, StagOp<T
     CSVisc1<T, 2> U;
     U.set(A, omega);
     const T* const alpha[2] = {A.alpha[0], A.alpha[1]};
-    t2_stag<T, NS>(nx, ny, blockIdx.x * t2_tx(NS), blockIdx.y * t2_ty(NS), R.src, R.dst, R.rhs, alpha, U, zero, sm);
+    t2_stag<T, NS, false>(nx, ny, blockIdx.x * t2_tx(NS), blockIdx.y * t2_ty(NS), R.src, R.dst, R.rhs, alpha, U, zero, true, sm);
 }
 
 template <typename T, int NS>
@@ -202,7 +222,7 @@ __global__ void __launch_bounds__(T2_THREADS) k_cc_t2(int nx, int ny, CCOp<T> A,
                                                       int zero) {
     __shared__ T sm[2 * 32 * T2_EY];
     t2_cc<T, NS, false>(nx, ny, blockIdx.x * t2_tx(NS), blockIdx.y * t2_ty(NS), src, dst, rhs, A.a[0], A.a[1], A.q,
-                        zero, sm);
+                        zero, true, sm);
 }
 
 inline dim3 t2_grid(const Grid& g, int ns) {
