@@ -1119,12 +1119,17 @@ int build(fhd_batch* B) {
         }
         // the coarse ends: the first level from which every coarser one fits
         // one CTA's shared memory (3 dim arrays per staggered level, 3 per
-        // pressure level)
+        // pressure level) and has at most 4096 cells (the largest box sets the
+        // pace of its launch: 128 boxes of 32^2 to 256^2, a step 21.2 ms with
+        // every level that fits, 20.4 with this limit, 20.7 with 2400).  Odd
+        // levels cannot go by launches.
         auto first = [&](int nl, const std::vector<Lev>& v, int per) {
             size_t acc = 0;
             int f = nl;
             for (int l = nl - 1; l >= 0; l--) {
                 acc += (size_t)per * (size_t)v[(size_t)b * MAXL + l].g.nc * sizeof(T);
+                const Grid& gl = v[(size_t)b * MAXL + l].g;
+                if (l < nl - 1 && gl.nc > 4096 && !(gl.n[0] & 1) && !(gl.n[1] & 1)) break;
                 if (acc > budget || nl - l > CS_MAXL) break;
                 f = l;
             }

@@ -845,16 +845,21 @@ static size_t coarse_smem_cap() {
 
 // first level of a hierarchy of n levels that the single-CTA coarse kernel
 // takes over (every level from it to the bottom fits the shared-memory
-// cap; level l needs bytes(l)); n when none does or the mode is off
-template <class F>
-static int coarse_first(fhd_ctx* ctx, int n, F bytes) {
+// cap; level l needs bytes(l)); n when none does or the mode is off.  Levels
+// above the bottom of more than max_cells go by launches although they would
+// fit: one SM takes longer than their 10 or so launches (measured whole
+// solves, us, with and without them: pressure 24^3 2012, 1640; 20^3 2070,
+// 1980; 2D 96^2 2048, 1800, 64^2 1718, 1640; 16^3 and 40^2 even; staggered 2D
+// 64^2 2910, 2780, 48^2 even).
+template <class C, class F>
+static int coarse_first(fhd_ctx* ctx, int n, i64 max_cells, C cells, F bytes) {
     if (ctx->coarse_mode == 0) return n;
     const size_t cap = coarse_smem_cap();
     size_t tot = 0;
     int lc = n;
     for (int l = n - 1; l >= 0 && n - l <= CS_MAXL; l--) {
         tot += bytes(l);
-        if (tot > cap) break;
+        if (tot > cap || (l < n - 1 && cells(l) > max_cells)) break;
         lc = l;
     }
     return lc;
@@ -865,13 +870,14 @@ static int stag_coarse_first(fhd_ctx* ctx, Multigrid<T>& M) {
     const int dim = ctx->dim;
     // the single-CTA coarse kernel knows walls for visc_type 1 only
     if (ctx->has_walls && ctx->visc != 1) return (int)M.s.size();
-    return coarse_first(ctx, (int)M.s.size(),
+    return coarse_first(ctx, (int)M.s.size(), dim == 2 ? 2400 : 1 << 20, [&](int l) { return M.s[l].g.nc; },
                         [&](int l) { return (size_t)(3 * dim) * (size_t)M.s[l].g.nc * sizeof(T); });
 }
 
 template <typename T>
 static int cc_coarse_first(fhd_ctx* ctx, Multigrid<T>& M) {
-    return coarse_first(ctx, (int)M.c.size(), [&](int l) { return (size_t)3 * (size_t)M.c[l].g.nc * sizeof(T); });
+    return coarse_first(ctx, (int)M.c.size(), ctx->dim == 2 ? 2400 : 4096, [&](int l) { return M.c[l].g.nc; },
+                        [&](int l) { return (size_t)3 * (size_t)M.c[l].g.nc * sizeof(T); });
 }
 
 // levels lc..bottom of the staggered V-cycle in one CTA: phi of level lc in
