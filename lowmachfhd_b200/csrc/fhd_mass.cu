@@ -836,22 +836,34 @@ __device__ __forceinline__ void d_stoch_face(const MixDev& m, int d, i64 f, cons
 // ---------------------------------------------------------------------
 // (FP32 with up to 4 species: a 64-register cap for 8 CTAs = 32 warps per
 // SM to hide the dependent chains)
+template <typename T>
+struct MassFluxArgs {
+    const double* rho[FHD_MAX_SPECIES];
+    const T* rwc;   // array (r, c) at (r * ns + c) * nc
+    const T* xc;    // array s at s * nc
+    T* flux;        // direction d, species s at (d * ns + s) * nc
+    const double* W[4 * 3 * FHD_MAX_SPECIES];
+    double wts[4];
+    int n_rngs;
+};
+
 template <typename T, int NS, int DIM>
 __global__ void __launch_bounds__(128, (sizeof(T) == 4 && NS <= 4) ? 8 : 1)
-    k_mass_flux(Grid g, MixDev m, int d, int wall, const double* const* __restrict__ rho,
-                const T* const* __restrict__ rwc, const T* const* __restrict__ xc,
-                const double* const* __restrict__ W, int n_rngs, const double* wts, T variance, T dxinv,
-                T* const* flux, TraceList tl) {
+    k_mass_flux(Grid g, MixDev m, int d, int wall, const __grid_constant__ MassFluxArgs<T> a, T variance, T dxinv,
+                TraceList tl) {
     Cell P;
     if (!cell_of_thread(g, P)) return;
-    const i64 f = P.id(0, 0, 0);
+    const i64 f = P.id(0, 0, 0), nc = g.nc;
+    T* const flux = a.flux + (i64)d * NS * nc;
+    auto xc = [&](int s, i64 i) { return ld(a.xc, s * nc + i); };
+    auto rwc = [&](int q, i64 i) { return ld(a.rwc, q * nc + i); };
     if (wall && (d == 0 ? P.i : (d == 1 ? P.j : P.k)) == 0) {
         // a wall face (wall: direction d has walls): the concentrations'
         // ghost cells are first-order extrapolated (scalar_bc,
         // inhomogeneous_bc_val.f90:21-54), so the diffusive flux vanishes,
         // and stoch_mass_bc zeroes the random field there
 #pragma unroll
-        for (int s = 0; s < NS; s++) flux[d * NS + s][f] = T(0);
+        for (int s = 0; s < NS; s++) flux[s * nc + f] = T(0);
         return;
     }
     const i64 fm = P.id(-(d == 0), -(d == 1), -(d == 2));
@@ -859,16 +871,16 @@ __global__ void __launch_bounds__(128, (sizeof(T) == 4 && NS <= 4) ? 8 : 1)
     {
         T gx[NS];
 #pragma unroll
-        for (int s = 0; s < NS; s++) gx[s] = (ld(xc[s], f) - ld(xc[s], fm)) * dxinv;
+        for (int s = 0; s < NS; s++) gx[s] = (xc(s, f) - xc(s, fm)) * dxinv;
 #pragma unroll
         for (int r = 0; r < NS; r++) {
             T acc = T(0);
 #pragma unroll
             for (int c = 0; c < NS; c++) {
                 if constexpr (sizeof(T) == 4)
-                    acc = __fmaf_rn(0.5f * (ld(rwc[r * NS + c], fm) + ld(rwc[r * NS + c], f)), gx[c], acc);
+                    acc = __fmaf_rn(0.5f * (rwc(r * NS + c, fm) + rwc(r * NS + c, f)), gx[c], acc);
                 else
-                    acc = acc + T(0.5) * (ld(rwc[r * NS + c], fm) + ld(rwc[r * NS + c], f)) * gx[c];
+                    acc = acc + T(0.5) * (rwc(r * NS + c, fm) + rwc(r * NS + c, f)) * gx[c];
             }
             fd[r] = acc;
         }
@@ -884,13 +896,13 @@ __global__ void __launch_bounds__(128, (sizeof(T) == 4 && NS <= 4) ? 8 : 1)
     for (int s = 0; s < NS; s++) fs[s] = T(0);
     if (m.var_mass != 0.0) {
         T ra[NS], rt;
-        d_face_rho_av<T, NS>(m, rho, f, fm, ra, rt);
+        d_face_rho_av<T, NS>(m, a.rho, f, fm, ra, rt);
         int na;
         d_active<T, NS>(m, ra, rt, &na);
         if (na == NS) {
             T L[NS][NS];
             d_sqrtL_full<T, NS>(m, ra, rt, L);
-            d_stoch_face<T, NS, DIM>(m, d, f, L, W, n_rngs, wts, variance, fs);
+            d_stoch_face<T, NS, DIM>(m, d, f, L, a.W, a.n_rngs, a.wts, variance, fs);
         } else if (na != 1) {
             // finished by k_mass_flux_trace, which adds the stochastic flux
             trace_push(tl, f);
@@ -898,7 +910,7 @@ __global__ void __launch_bounds__(128, (sizeof(T) == 4 && NS <= 4) ? 8 : 1)
         // na == 1: zero factor, no stochastic flux
     }
 #pragma unroll
-    for (int s = 0; s < NS; s++) flux[d * NS + s][f] = fd[s] + fs[s];
+    for (int s = 0; s < NS; s++) flux[s * nc + f] = fd[s] + fs[s];
 }
 
 // the listed faces of k_mass_flux: the stochastic flux through the
@@ -1117,13 +1129,21 @@ static int mass_fluxdiv_T(fhd_ctx* ctx, MassBufs& B, const MixDev& m, const doub
     FHD_CUDA_TRY(cudaPeekAtLastError());
     const T variance = (T)sqrt(2.0 * m.kB * m.var_mass / (m.dV * dt));
     const T dxinv = (T)(1.0 / ctx->dx);
+    MassFluxArgs<T> fa;
+    memset(&fa, 0, sizeof(fa));
+    for (int s = 0; s < NS; s++) fa.rho[s] = rho[s];
+    for (int q = 0; q < n_rngs * dim * NS; q++) fa.W[q] = W[q];
+    for (int r = 0; r < n_rngs; r++) fa.wts[r] = weights[r];
+    fa.rwc = (const T*)B.rwc;
+    fa.xc = (const T*)B.xc;
+    fa.flux = (T*)B.flux;
+    fa.n_rngs = n_rngs;
     for (int d = 0; d < dim; d++) {
         FHD_CUDA_TRY(cudaMemsetAsync(B.tl.count, 0, sizeof(unsigned), st));
         with_dim(dim, [&](auto D) {
             constexpr int DIM = decltype(D)::value;
             k_mass_flux<T, NS, DIM><<<dim3((g.n[0] + 31) / 32, (g.n[1] + 3) / 4, g.n[2]), dim3(32, 4, 1), 0, st>>>(
-                g, m, d, ctx->has_walls && ctx->walls.lo[d] != 0, d_rho, (const T* const*)d_rwc, (const T* const*)d_xc,
-                d_W, n_rngs, B.wts, variance, dxinv, d_flux, B.tl);
+                g, m, d, ctx->has_walls && ctx->walls.lo[d] != 0, fa, variance, dxinv, B.tl);
             k_mass_flux_trace<T, NS, DIM><<<nbt, 128, 0, st>>>(g, m, d, d_rho, d_W, n_rngs, B.wts, variance, d_flux,
                                                                B.tl);
         });
