@@ -1702,6 +1702,26 @@ static int cc_solve(fhd_ctx* ctx, Multigrid<T>& M) {
     return rc;
 }
 
+static CSVec<double> csv(SVec<double> v) {
+    CSVec<double> o;
+    for (int c = 0; c < 4; c++) o.c[c] = v.c[c];
+    return o;
+}
+
+static int gs_blocks(i64 nc) {
+    const int b = flat_blocks(nc);
+    return b < GS_BLOCKS ? b : GS_BLOCKS;
+}
+
+// f(NV) with NV = nv as a constant, 1 <= nv <= GS_MAXV
+template <int N = GS_MAXV, class F>
+static void with_nv(int nv, F&& f) {
+    if constexpr (N > 1) {
+        if (nv < N) return with_nv<N - 1>(nv, f);
+    }
+    f(std::integral_constant<int, N>());
+}
+
 // ---------------------------------------------------------------------
 // apply_precon (apply_precon.f90:29-475); visc_schur_approx 0 (simple
 // Schur complements) or 1 (visc_schur_complement, 538-685)
@@ -1731,23 +1751,18 @@ static int precon_T(fhd_ctx* ctx, CSVec<double> b, SVec<double> x) {
     // starts from zero
     for (int c = 0; c < dim; c++) L0.phi[c] = fp64 ? (T*)x.c[c] : M.x_u[c];
     auto set_rhs_from_b = [&]() -> int {
-        for (int c = 0; c < dim; c++) {
-            if (fp64) {
-                L0.rhs[c] = (T*)b.c[c];
-            } else {
-                k_copy_conv<T, double><<<nb, 256, 0, st>>>(nc, M.b_u[c], b.c[c], 1.0);
-                FHD_POST(ctx);
-                L0.rhs[c] = M.b_u[c];
-            }
-        }
+        for (int c = 0; c < dim; c++) L0.rhs[c] = fp64 ? (T*)b.c[c] : M.b_u[c];
+        if (fp64) return 0;
+        const SVec<T> o = {{M.b_u[0], M.b_u[1], M.b_u[2], nullptr}};
+        with_dim(dim, [&](auto D) { k_convs<T, double, decltype(D)::value><<<nb, 256, 0, st>>>(nc, o, b); });
+        FHD_POST(ctx);
         return 0;
     };
     auto phi_to_x = [&]() -> int {
         if (fp64) return 0;
-        for (int c = 0; c < dim; c++) {
-            k_copy_conv<double, T><<<nb, 256, 0, st>>>(nc, x.c[c], L0.phi[c], 1.0);
-            FHD_POST(ctx);
-        }
+        const CSVec<T> in = {{L0.phi[0], L0.phi[1], L0.phi[2], nullptr}};
+        with_dim(dim, [&](auto D) { k_convs<double, T, decltype(D)::value><<<nb, 256, 0, st>>>(nc, x, in); });
+        FHD_POST(ctx);
         return 0;
     };
     auto div_plus = [&](const double* bp) -> int {
@@ -1896,21 +1911,20 @@ static int precon_T(fhd_ctx* ctx, CSVec<double> b, SVec<double> x) {
     }
     // null space: mean of p, and of u when theta_alpha = 0 and no wall is
     // no-slip, for the periodic directions -- apply_precon.f90:429-460
-    k_sum<double><<<nb, RED_THREADS, 0, st>>>(nc, x.c[dim], slot(ctx, S_MEAN));
-    FHD_POST(ctx);
-    k_sub_mean<double><<<nb, 256, 0, st>>>(nc, x.c[dim], ctx->dscal + S_MEAN, (double)nc);
-    FHD_POST(ctx);
-    if (theta == 0.0 && !ctx->noslip) {
-        for (int c = 0; c < dim; c++) {
-            // the velocity means go for periodic directions only
-            if (ctx->walls.lo[c] != 0) continue;
-            k_sum<double><<<nb, RED_THREADS, 0, st>>>(nc, x.c[c], slot(ctx, S_MEAN + 1 + c));
-            FHD_POST(ctx);
-            k_sub_mean<double><<<nb, 256, 0, st>>>(nc, x.c[c], ctx->dscal + S_MEAN + 1 + c, (double)nc);
-            FHD_POST(ctx);
-        }
-    }
-    return 0;
+    SVec<double> z = {{x.c[dim], nullptr, nullptr, nullptr}};
+    int nz = 1;
+    if (theta == 0.0 && !ctx->noslip)
+        for (int c = 0; c < dim; c++)
+            if (ctx->walls.lo[c] == 0) z.c[nz++] = x.c[c];  // the velocity means go for periodic directions only
+    with_nv<4>(nz, [&](auto N) {
+        constexpr int NZ = decltype(N)::value;
+        k_sums<NZ><<<gs_blocks(nc), RED_THREADS, 0, st>>>(nc, csv(z), ctx->dscal + S_MEAN, ctx->gs.partials,
+                                                         ctx->gs.counter);
+        rc |= post(ctx);
+        k_sub_means<NZ><<<nb, 256, 0, st>>>(nc, z, ctx->dscal + S_MEAN, (double)nc);
+        rc |= post(ctx);
+    });
+    return rc;
 }
 
 int precon(fhd_ctx* ctx, CSVec<double> b, SVec<double> x) {
@@ -2169,17 +2183,6 @@ static SVec<double> svec(double* base, int dim, i64 nc) {
     for (int c = 0; c < 4; c++) v.c[c] = c <= dim ? base + (i64)c * nc : nullptr;
     return v;
 }
-static CSVec<double> csv(SVec<double> v) {
-    CSVec<double> o;
-    for (int c = 0; c < 4; c++) o.c[c] = v.c[c];
-    return o;
-}
-
-static int gs_blocks(i64 nc) {
-    const int b = flat_blocks(nc);
-    return b < GS_BLOCKS ? b : GS_BLOCKS;
-}
-
 // |a|^2 into a scalar slot, and its inverse root where asked
 static int wnorm2(fhd_ctx* ctx, CSVec<double> a, int slotid, double* inv = nullptr) {
     const i64 nc = ctx->g0.nc;
@@ -2189,15 +2192,6 @@ static int wnorm2(fhd_ctx* ctx, CSVec<double> a, int slotid, double* inv = nullp
             nc, a, wp * wp, ctx->dscal + slotid, inv, ctx->gs.partials, ctx->gs.counter);
     });
     return post(ctx);
-}
-
-// f(NV) with NV = nv as a constant, 1 <= nv <= GS_MAXV
-template <int N = GS_MAXV, class F>
-static void with_nv(int nv, F&& f) {
-    if constexpr (N > 1) {
-        if (nv < N) return with_nv<N - 1>(nv, f);
-    }
-    f(std::integral_constant<int, N>());
 }
 
 // the new Krylov vector w orthogonalised against u_0 .. u_{i-1}, as u_i

@@ -71,14 +71,6 @@ __device__ __forceinline__ void red_finish(double v, RedSlot rs) {
     }
 }
 
-// sum_f a[f]
-template <typename T>
-static __global__ void __launch_bounds__(RED_THREADS) k_sum(i64 n, const T* a, RedSlot rs) {
-    double s = 0.0;
-    for (i64 f = blockIdx.x * (i64)blockDim.x + threadIdx.x; f < n; f += (i64)gridDim.x * blockDim.x) s += (double)a[f];
-    red_finish(s, rs);
-}
-
 // ---------------------------------------------------------------------
 // Orthogonalisation of a new Krylov vector w against i others
 // (gmres.f90:352-389), two passes over the vectors instead of one per
@@ -173,6 +165,34 @@ static __global__ void __launch_bounds__(RED_THREADS, 4) k_norm2(i64 n, CSVec<do
     if (!red_many<1>(s, partials, counter, tot) || threadIdx.x) return;
     *out = tot[0];
     if (inv) *inv = 1.0 / sqrt(tot[0]);
+}
+
+// sums of the N fields of a into out[0 .. N), in one pass (one launch for the
+// null space of the preconditioner: a 64^2 field's sum costs its launch, 3.3 us
+// each one by one)
+template <int N>
+static __global__ void __launch_bounds__(RED_THREADS, 4) k_sums(i64 n, CSVec<double> a, double* out, double* partials,
+                                                                unsigned* counter) {
+    double s[N];
+#pragma unroll
+    for (int c = 0; c < N; c++) s[c] = 0.0;
+    for (i64 f = blockIdx.x * (i64)blockDim.x + threadIdx.x; f < n; f += (i64)gridDim.x * blockDim.x)
+#pragma unroll
+        for (int c = 0; c < N; c++) s[c] += a.c[c][f];
+    __shared__ double tot[N];
+    if (!red_many<N>(s, partials, counter, tot)) return;
+    if (threadIdx.x < N) out[threadIdx.x] = tot[threadIdx.x];
+}
+
+// the fields less their means sum[c] / count
+template <int N>
+static __global__ void __launch_bounds__(256) k_sub_means(i64 n, SVec<double> a, const double* sum, double count) {
+    double m[N];
+#pragma unroll
+    for (int c = 0; c < N; c++) m[c] = sum[c] / count;
+    for (i64 f = blockIdx.x * (i64)blockDim.x + threadIdx.x; f < n; f += (i64)gridDim.x * blockDim.x)
+#pragma unroll
+        for (int c = 0; c < N; c++) a.c[c][f] = a.c[c][f] - m[c];
 }
 
 // <w, u_k> and <u_{i-1}, u_k> for k = k0 .. k0 + NV - 1; the last block of the
@@ -285,6 +305,19 @@ static __global__ void __launch_bounds__(256) k_update_sol(i64 n, int ncomp, SVe
     }
 }
 
+// N fields converted in one launch (the velocity between GMRES and the FP32
+// multigrid)
+template <typename TO, typename TI, int N>
+static __global__ void __launch_bounds__(256) k_convs(i64 n, SVec<TO> o, CSVec<TI> in) {
+    for (i64 f = blockIdx.x * (i64)blockDim.x + threadIdx.x; f < n; f += (i64)gridDim.x * blockDim.x) {
+        TI v[N];
+#pragma unroll
+        for (int c = 0; c < N; c++) v[c] = in.c[c][f];
+#pragma unroll
+        for (int c = 0; c < N; c++) o.c[c][f] = (TO)v[c];
+    }
+}
+
 template <typename TO, typename TI>
 static __global__ void __launch_bounds__(256) k_copy_conv(i64 n, TO* __restrict__ o, const TI* __restrict__ in, double s) {
     // four grid strides per pass: four loads in flight per thread
@@ -298,13 +331,6 @@ static __global__ void __launch_bounds__(256) k_copy_conv(i64 n, TO* __restrict_
         for (int u = 0; u < 4; u++) o[f + u * st] = (TO)((double)a[u] * s);
     }
     for (; f < n; f += st) o[f] = (TO)((double)in[f] * s);
-}
-
-template <typename T>
-static __global__ void __launch_bounds__(256) k_sub_mean(i64 n, T* a, const double* sum, double count) {
-    const double m = (*sum) / count;
-    for (i64 f = blockIdx.x * (i64)blockDim.x + threadIdx.x; f < n; f += (i64)gridDim.x * blockDim.x)
-        a[f] = (T)((double)a[f] - m);
 }
 
 template <typename T>
