@@ -197,16 +197,17 @@ int  fhd_ctx_set_stream(fhd_ctx* ctx, void* stream);
 int fhd_ctx_set_graphs(fhd_ctx* ctx, int mode);
 /* The coarse end of both multigrid V-cycles (every level from the first
  * whose unknowns, right-hand sides and residuals fit in one SM's shared
- * memory down to the bottom) as one single-block kernel per V-cycle instead
- * of one launch per smoother colour and transfer (mode 1 or -1 default: on,
- * 0: per-level launches).  Same arithmetic either way.  Replaces no
+ * memory down to the bottom, up to the sizes where launches are faster) as one
+ * single-block kernel per V-cycle instead of one launch per smoother colour
+ * and transfer (mode 1 or -1 default: on, 0: per-level launches).  Same arithmetic either way.  Replaces no
  * reference routine: the levels are those of stag_mg_solver.f90:301-599 and
  * of the pressure multigrid behind macproject.f90:294-298. */
 int fhd_ctx_set_coarse(fhd_ctx* ctx, int mode);
-/* Whole smooths (both colours of every component) of the large FP32 levels
- * of a visc_type 1 staggered multigrid as one row-tile launch each, staged
- * by the bulk-copy engine, instead of one launch per colour (mode 1 or -1
- * default: on where the level allows, 0: colour launches).  The colour
+/* Whole smooths (both colours of every component, one or two smooths per
+ * launch) of the levels of even extents, instead of one launch per colour: 3D
+ * visc_type 1 staggered levels by a march in z, 2D visc_type 1 staggered and
+ * pressure levels on tiles (mode 1 or -1 default: on where the level allows,
+ * 0: colour launches).  The colour
  * sweeps of stag_mg_solver.f90:360-396, evaluated in the same order. */
 int fhd_ctx_set_fused(fhd_ctx* ctx, int mode);
 /* Moving no-slip walls: the namelist arrays wallspeed_lo / wallspeed_hi of
@@ -232,7 +233,8 @@ int fhd_ctx_set_wall_speed(fhd_ctx* ctx, const double wallspeed_lo[6], const dou
  * tiled fused smooth with one of several tile sizes (3D), or as the row-tile
  * smooth with one of the tile heights that fit, one CTA per SM with a deep
  * copy ring (256 or 512 compute threads) or two with a short one (3D FP32
- * visc_type 1).  With
+ * visc_type 1).  Levels that fhd_ctx_set_fused's march or tiles take use
+ * those, one past the candidate list, timed for the record only.  With
  * the tuner on (mode 1 or -1 default), the first solve call that meets a
  * level shape times every candidate on scratch unknowns with the level's
  * coefficients and keeps the fastest for the process (per device,

@@ -593,7 +593,7 @@ __global__ void __launch_bounds__(256) kb_stokes_apply(const Tile* tiles, int n,
     });
 }
 
-// Modified Gram-Schmidt pass k (k_mgs): w -= h[k-1] V_{k-2} (k > 1), then
+// Modified Gram-Schmidt pass k: w -= h[k-1] V_{k-2} (k > 1), then
 // the tile's partial of <w, V_{k-1}> (or <w, w> when vnext is null)
 __global__ void __launch_bounds__(256) kb_mgs(const Tile* tiles, int n, const Lev* lev, const Ctl* ctl, double* const* w,
                                               const double* const* vprev, int hk, const double* const* vnext,
@@ -629,8 +629,8 @@ __global__ void __launch_bounds__(256) kb_mgs(const Tile* tiles, int n, const Le
     });
 }
 
-// v = w / |w| with |w| = sqrt(ctl.h[hk]) (k_scale_by_norm), or w / norm_resid
-// (k_scale_div, hk < 0)
+// v = w / |w| with |w| = sqrt(ctl.h[hk]) , or w / norm_resid
+// (hk < 0)
 __global__ void __launch_bounds__(256) kb_scale(const Tile* tiles, int n, const Lev* lev, const Ctl* ctl,
                                                 double* const* v, const double* const* w, int hk) {
     for_tiles(tiles, n, ctl, M_INNER, [&](const Tile& t, int q) {
