@@ -246,11 +246,12 @@ int fhd_ctx_set_wall_speed(fhd_ctx* ctx, const double wallspeed_lo[6], const dou
  * macproject multigrid) in the same order; the choice changes time only. */
 int fhd_ctx_set_tune(fhd_ctx* ctx, int mode);
 /* Plan of staggered (which 0) or pressure (which 1) multigrid level `level`
- * after the last solve call: kind -1 fixed rules, 0 colour launches, 1 tiled
- * fused, 2 row-tile; ncand candidates considered; pair_us the measured time
- * of one smooth pair (0 when not timed); shape = {block x, block y, 0, 1,
- * threads} for colour launches, {tile x, tile y, z-runs, CTAs per SM,
- * compute threads} for fused smooths.  Any output pointer may be NULL.  No
+ * after the last solve call: kind -1 fixed rules, 0 colour launches, 1 fused
+ * smooths (tiled; the march and the 2D tiles of fhd_ctx_set_fused, with the
+ * shape of their two smooths per launch), 2 row-tile; ncand candidates
+ * considered; pair_us the measured time of one smooth pair (0 when not
+ * timed); shape = {block x, block y, 0, 1, threads} for colour launches,
+ * {tile x, tile y, z-runs, CTAs per SM, compute threads} for fused smooths.  Any output pointer may be NULL.  No
  * reference counterpart. */
 int fhd_ctx_tune_info(fhd_ctx* ctx, int which, int level, int* kind, int* ncand, double* pair_us,
                       int shape[5]);

@@ -147,7 +147,7 @@ class StokesSolver:
 
     def tune_info(self, which: str = "stag", level: int = 0) -> dict:
         """plan of one level after the last solve call: kind (-1 fixed rules,
-        0 colour launches, 1 tiled fused, 2 row-tile), candidates considered,
+        0 colour launches, 1 fused -- tiles or march --, 2 row-tile), candidates considered,
         measured time of a smooth pair, block or tile shape"""
         kind, nc, us = C.c_int(0), C.c_int(0), C.c_double(0)
         shape = (C.c_int * 5)()

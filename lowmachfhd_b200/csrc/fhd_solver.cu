@@ -2845,18 +2845,22 @@ int fhd_ctx_tune_info(fhd_ctx* c, int which, int level, int* kind, int* ncand, d
     if (ncand) *ncand = P->ncand;
     if (pair_us) *pair_us = P->us;
     if (shape) {
-        const ZMGeom* Z = P->march ? (c->prec == FHD_PREC_MIXED ? &c->mg32.s[level].zm[1] : &c->mg64.s[level].zm[1])
-                                   : nullptr;
         shape[0] = P->kind == 0 ? P->bx : P->kind == 1 ? P->rb.TX : P->kind == 2 ? c->n[0] : 0;
         shape[1] = P->kind == 0 ? P->by : P->kind == 1 ? P->rb.TY : P->kind == 2 ? P->rbx.TY : 0;
         shape[2] = P->kind == 1 ? P->rb.chunks : P->kind == 2 ? P->rbx.chunks : 0;
         shape[3] = P->kind == 2 ? P->rbx.per_sm : P->kind >= 0 ? 1 : 0;
         shape[4] = P->kind == 0 ? P->bx * P->by : P->kind == 1 ? P->rb.threads : P->kind == 2 ? P->rbx.threads : 0;
-        if (Z) {
-            shape[0] = 2 * Z->ip;
-            shape[1] = Z->TY;
-            shape[2] = Z->chunks;
-            shape[4] = Z->threads;
+        if (P->march && c->dim == 2) {  // the tiles of fhd_t2.cuh, of either multigrid
+            shape[0] = t2_tx(2);
+            shape[1] = t2_ty(2);
+            shape[2] = 1;
+            shape[4] = T2_THREADS;
+        } else if (P->march) {  // the z-march: staggered levels only
+            const ZMGeom& Z = c->prec == FHD_PREC_MIXED ? c->mg32.s[level].zm[1] : c->mg64.s[level].zm[1];
+            shape[0] = 2 * Z.ip;
+            shape[1] = Z.TY;
+            shape[2] = Z.chunks;
+            shape[4] = Z.threads;
         }
     }
     return FHD_OK;
