@@ -652,17 +652,21 @@ static int stag_smooths_planned(fhd_ctx* ctx, StagLevel<T>& L, const SmoothPlan&
     return 0;
 }
 
-// whether a level smooths with the z-march (3D, even extents of at least four
-// cells) or on tiles (2D, even extents: fhd_t2.cuh): constant viscosity
-// without cross terms; not where a caller
-// forced or imported a plan, or asked for colour launches (fhd_ctx_set_fused
-// 0).  It is the fastest form at every size it takes (a pair of smooths,
-// FP32, before and now: 40^3 52 -> 9 us, 128^3 64 -> 44, 192^3 238 -> 113,
-// 256^3 349 -> 280; FP64 128^3 136 -> 99), so no plan is timed against it.
+// zm_use: whether a level smooths with the z-march (3D, even extents of at least
+// four cells) or on tiles (2D, even extents: fhd_t2.cuh): constant viscosity
+// without cross terms (zm_shape, all that the process's plan table may go by);
+// not where a caller forced or imported a plan, or asked for colour launches
+// (fhd_ctx_set_fused 0), or where an array is not aligned.  It is the fastest
+// form at every size it takes (a pair of smooths, FP32, before and now: 40^3
+// 52 -> 9 us, 128^3 64 -> 44, 192^3 238 -> 113, 256^3 349 -> 280; FP64 128^3
+// 136 -> 99), so no plan is timed against it.
+template <typename T>
+static bool zm_shape(fhd_ctx* ctx, const StagLevel<T>& L) {
+    return L.zm_ok && ctx->visc == 1 && ctx->p.stag_mg_smoother != 0 && !ctx->has_walls;
+}
 template <typename T>
 static bool zm_use(fhd_ctx* ctx, const StagLevel<T>& L) {
-    return L.zm_ok && ctx->visc == 1 && ctx->fused_mode != 0 && ctx->p.stag_mg_smoother != 0 && !ctx->has_walls &&
-           (L.plan.kind < 0 || L.plan.march) && stag_aligned(L, ctx->dim);
+    return zm_shape(ctx, L) && ctx->fused_mode != 0 && (L.plan.kind < 0 || L.plan.march) && stag_aligned(L, ctx->dim);
 }
 
 // one launch of ns smooths phi -> tmp of every component; the two buffers
@@ -1199,15 +1203,19 @@ static int cc_rb_pairs(fhd_ctx* ctx, CCLevel<T>& C, const RBGeom& G, int pairs) 
     return 0;
 }
 
-// whether a level smooths on tiles (fhd_t2.cuh): 2D, even extents; not where a
-// caller forced or imported a plan, or asked for colour launches
-// (fhd_ctx_set_fused 0).  One launch in place of four, at every size in use: no
-// plan is timed against it.
+// cc_t2_use: whether a level smooths on tiles (fhd_t2.cuh): 2D, even extents
+// (cc_t2_shape, all that the process's plan table may go by); not where a caller
+// forced or imported a plan, or asked for colour launches (fhd_ctx_set_fused
+// 0).  One launch in place of four, at every size in use: no plan is timed
+// against it.
+template <typename T>
+static bool cc_t2_shape(const CCLevel<T>& C) {
+    return C.g.dim == 2 && all_even(C.g) && C.g.nc < (1ll << 31);
+}
 template <typename T>
 static bool cc_t2_use(fhd_ctx* ctx, const CCLevel<T>& C) {
-    return ctx->dim == 2 && all_even(C.g) && C.g.nc < (1ll << 31) && ctx->fused_mode != 0 &&
-           (C.plan.kind < 0 || C.plan.march) && rb_aligned(C.phi) && rb_aligned(C.tmp) && rb_aligned(C.rhs) &&
-           rb_aligned(C.a[0]) && rb_aligned(C.a[1]);
+    return cc_t2_shape(C) && ctx->fused_mode != 0 && (C.plan.kind < 0 || C.plan.march) && rb_aligned(C.phi) &&
+           rb_aligned(C.tmp) && rb_aligned(C.rhs) && rb_aligned(C.a[0]) && rb_aligned(C.a[1]);
 }
 
 // one launch of ns smooths phi -> tmp; the two buffers then change names
@@ -1431,7 +1439,7 @@ static int tune_levels_locked(fhd_ctx* ctx, Multigrid<T>& M, std::vector<T*>& sc
         march.march = true;
         march.ncand = nlist;
         march.index = nlist;
-        const bool can_march = zm_use(ctx, L);
+        const bool can_march = zm_shape(ctx, L);
         if (force >= 0) {
             if (force == nlist && can_march) {
                 L.plan = march;
@@ -1497,7 +1505,7 @@ static int tune_levels_locked(fhd_ctx* ctx, Multigrid<T>& M, std::vector<T*>& sc
         march.march = true;
         march.ncand = nlist;
         march.index = nlist;
-        const bool can_march = cc_t2_use(ctx, C);
+        const bool can_march = cc_t2_shape(C);
         if (force >= 0) {
             if (force == nlist && can_march) {
                 C.plan = march;
@@ -1515,6 +1523,9 @@ static int tune_levels_locked(fhd_ctx* ctx, Multigrid<T>& M, std::vector<T*>& sc
             g_tune[key] = C.plan;
             continue;
         }
+        // asked for colour launches where the shape takes the tiles: the fixed
+        // rules, as a plan timed without the tiles is not the shape's
+        if (can_march && ctx->fused_mode == 0) continue;
         if (int rc = get_scratch(nc_max)) return rc;
         CCLevel<T> S = C;
         S.phi = scratch[0];
