@@ -851,9 +851,9 @@ static size_t coarse_smem_cap() {
 // takes over (every level from it to the bottom fits the shared-memory
 // cap; level l needs bytes(l)); n when none does or the mode is off.  Levels
 // above the bottom of more than max_cells go by launches although they would
-// fit: one SM takes longer than their 10 or so launches (measured whole
-// solves, us, with and without them: pressure 24^3 2012, 1640; 20^3 2070,
-// 1980; 2D 96^2 2048, 1800, 64^2 1718, 1640; 16^3 and 40^2 even; staggered 2D
+// fit: one SM takes longer than their launches (measured whole solves, us,
+// with and without them: pressure 24^3 2012, 1640; 20^3 2070, 1980; 2D 96^2
+// 2048, 1800, 64^2 1718, 1640; 16^3 and 40^2 even; staggered 2D visc_type 1
 // 64^2 2910, 2780, 48^2 even).
 template <class C, class F>
 static int coarse_first(fhd_ctx* ctx, int n, i64 max_cells, C cells, F bytes) {
@@ -874,7 +874,14 @@ static int stag_coarse_first(fhd_ctx* ctx, Multigrid<T>& M) {
     const int dim = ctx->dim;
     // the single-CTA coarse kernel knows walls for visc_type 1 only
     if (ctx->has_walls && ctx->visc != 1) return (int)M.s.size();
-    return coarse_first(ctx, (int)M.s.size(), dim == 2 ? 2400 : 1 << 20, [&](int l) { return M.s[l].g.nc; },
+    // 2D limit by type, whole solves in us without a limit, with 2400 and with
+    // 4096 cells: visc_type -1 FP32 (components swept together) 48 x 64 1717,
+    // 1848, 1726, 64^2 1751, 1836, 1752, 128^2 2253, 2361, 2256; 72^2 1889,
+    // 1804 and 80^2 2202, 1946 without and with.  The others gain by 2400: -1
+    // FP64 56^2 2023, 1876; 2 64^2 1899, 1812; -2 56^2 1967, 1814; 3 64^2 1926,
+    // 1881; -3 64^2 2342, 2221; 1 with walls 56^2 1968, 1927 (FP32), 2166, 2045.
+    const int lim2 = ctx->visc == -1 && std::is_same<T, float>::value ? 4096 : 2400;
+    return coarse_first(ctx, (int)M.s.size(), dim == 2 ? lim2 : 1 << 20, [&](int l) { return M.s[l].g.nc; },
                         [&](int l) { return (size_t)(3 * dim) * (size_t)M.s[l].g.nc * sizeof(T); });
 }
 
