@@ -135,20 +135,33 @@ struct Sched {
 static uint64_t request_bytes(const fhd_request* r) {
     const int dim = r->dim, nE = dim == 2 ? 1 : 3, ns = r->nspecies;
     uint64_t nc = 1;
-    for (int d = 0; d < dim; d++) nc *= (uint64_t)r->n_cells[d];
+    bool odd = false;
+    for (int d = 0; d < dim; d++) {
+        nc *= (uint64_t)r->n_cells[d];
+        odd = odd || (r->n_cells[d] & 1);
+    }
     const int m = r->params.gmres_max_inner;
-    const double s = r->precision == FHD_PREC_MIXED ? 4.0 : 8.0;
-    // multigrid: per level phi, rhs, tmp, alpha (dim each), beta, gamma,
-    // edges, in mixed 3D the row-tile smoother's diagonal (dim); cc: a (dim),
-    // phi, rhs, tmp; level sums to 8/7 (3D) or 4/3 (2D)
-    const double lv = dim == 3 ? 8.0 / 7.0 : 4.0 / 3.0;
-    const double rbx = (r->precision == FHD_PREC_MIXED && dim == 3) ? dim : 0;
-    const double mg = (4.0 * dim + 2 + nE + dim + 3 + 2 * dim + 1 + rbx) * s * lv;
-    const double krylov = (double)(m + 1 + 4) * (dim + 1) * 8.0;
+    const bool mixed = r->precision == FHD_PREC_MIXED, bfbt = r->params.visc_schur_approx != 0;
+    const double s = mixed ? 4.0 : 8.0;
+    // multigrid (build_mg): the finest level's tmp (dim), in the mixed mode its
+    // copies of alpha (dim), beta, gamma and the edges, the two-pass smoother's
+    // diagonal (dim) of an odd extent or the Jacobi smoother; the pressure level's
+    // a (dim), phi, rhs, tmp; x_u, b_u (dim each), mac_rhs
+    const bool jacobi = r->params.stag_mg_smoother == 0;
+    const double fine = dim + (mixed ? dim + 2 + nE : 0) + (odd || jacobi ? dim : 0) + dim + 3 + 2 * dim + 1 +
+                        (bfbt ? 2 * dim + 1 : 0);
+    // every coarser level, together 1/7 (3D) or 1/3 (2D) of the finest: phi, rhs,
+    // tmp, alpha, diagonal (dim each), beta, gamma, edges; a, phi, rhs, tmp
+    const double coarse = (5.0 * dim + 2 + nE + dim + 3 + (bfbt ? dim : 0)) / (dim == 3 ? 7.0 : 3.0);
+    // the autotuner's scratch of the finest level, held while the first request of
+    // a shape prepares
+    const double mg = (fine + coarse + 3.0 * dim) * s;
+    // V (m + 1 vectors), w, tmp, xs
+    const double krylov = (double)(m + 1 + 3) * (dim + 1) * 8.0;
     const double step = (39.0 + ns * (2 + dim)) * 8.0;
-    const double mass = ns > 1 ? (ns * ns + ns + dim * ns) * s : 0.0;
+    const double mass = ns > 1 ? (ns * ns + ns + dim * ns) * s + 4.0 : 0.0;
     const double state = (dim + ns + 1 + 1 + nE + 1 + 1 + nE + ns) * 8.0;
-    const double noise = (2.0 * dim + 2.0 * nE + 2.0 * dim * ns) * 8.0;
+    const double noise = (2.0 * dim + 2.0 * nE + (ns > 1 ? 2.0 * dim * ns : 0.0)) * 8.0;
     return (uint64_t)((mg + krylov + step + mass + state + noise) * (double)nc) + (64ull << 20);
 }
 
