@@ -834,8 +834,6 @@ __device__ __forceinline__ void d_stoch_face(const MixDev& m, int d, i64 f, cons
 // per face of direction D (the low face of each cell): diffusive +
 // stochastic flux, corrected (correction_flux.f90:17-226)
 // ---------------------------------------------------------------------
-// (FP32 with up to 4 species: a 64-register cap for 8 CTAs = 32 warps per
-// SM to hide the dependent chains)
 template <typename T>
 struct MassFluxArgs {
     const double* rho[FHD_MAX_SPECIES];
@@ -847,8 +845,19 @@ struct MassFluxArgs {
     int n_rngs;
 };
 
+// Blocks of 128 threads per SM that the registers are capped for, to have more
+// warps hide the dependent chains: FP32 with up to 4 species 8 (64 registers; 189
+// -> 164 us per direction at 128^3); FP64 with 3 species 5 (92 registers, no
+// spills): since the pointers are parameters the uncapped kernel takes 106 and is
+// scheduled worse (whole calls at 128^3: pointers from a device table 1151 us,
+// parameters uncapped 1265, capped 1131).
+template <typename T>
+constexpr int mass_flux_blocks(int ns) {
+    return sizeof(T) == 4 ? (ns <= 4 ? 8 : 1) : ns == 3 ? 5 : 1;
+}
+
 template <typename T, int NS, int DIM>
-__global__ void __launch_bounds__(128, (sizeof(T) == 4 && NS <= 4) ? 8 : 1)
+__global__ void __launch_bounds__(128, mass_flux_blocks<T>(NS))
     k_mass_flux(Grid g, MixDev m, int d, int wall, const __grid_constant__ MassFluxArgs<T> a, T variance, T dxinv,
                 TraceList tl) {
     Cell P;
