@@ -869,25 +869,33 @@ static int coarse_first(fhd_ctx* ctx, int n, i64 max_cells, C cells, F bytes) {
     return lc;
 }
 
+// (graph: the launches are replayed as a graph.  Outside one a launch costs 3 to
+// 4 us instead of 1.7, and levels that smooth by colour launches enter the kernel
+// as soon as they fit: stag_mg_solver calls, visc_type 2, with and without them
+// as launches, 64^2 FP32 295, 267, 256 x 192 FP32 480, 444, FP64 445, 415.)
+constexpr i64 CS_NO_LIMIT = 1 << 20;
+
 template <typename T>
-static int stag_coarse_first(fhd_ctx* ctx, Multigrid<T>& M) {
+static int stag_coarse_first(fhd_ctx* ctx, Multigrid<T>& M, bool graph) {
     const int dim = ctx->dim;
     // the single-CTA coarse kernel knows walls for visc_type 1 only
     if (ctx->has_walls && ctx->visc != 1) return (int)M.s.size();
     // 2D limit by type, whole solves in us without a limit, with 2400 and with
-    // 4096 cells: visc_type -1 FP32 (components swept together) 48 x 64 1717,
-    // 1848, 1726, 64^2 1751, 1836, 1752, 128^2 2253, 2361, 2256; 72^2 1889,
+    // 4096 cells: visc_type -1 FP32 (components swept together) 48 x 64 1607,
+    // 1721, 1607, 64^2 1721, 1735, 1714, 128^2 2163, 2225, 2173; 72^2 1889,
     // 1804 and 80^2 2202, 1946 without and with.  The others gain by 2400: -1
-    // FP64 56^2 2023, 1876; 2 64^2 1899, 1812; -2 56^2 1967, 1814; 3 64^2 1926,
-    // 1881; -3 64^2 2342, 2221; 1 with walls 56^2 1968, 1927 (FP32), 2166, 2045.
-    const int lim2 = ctx->visc == -1 && std::is_same<T, float>::value ? 4096 : 2400;
-    return coarse_first(ctx, (int)M.s.size(), dim == 2 ? lim2 : 1 << 20, [&](int l) { return M.s[l].g.nc; },
+    // FP64 56^2 2023, 1876; 2 64^2 1899, 1812; -2 56^2 1967, 1814; 3 64^2 1875,
+    // 1767; -3 64^2 2145, 2071; 1 with walls 56^2 1895, 1888 (FP32), 2058, 2018.
+    const bool whole = ctx->has_walls || (ctx->visc == 1 && ctx->p.stag_mg_smoother != 0 && ctx->fused_mode != 0);
+    const i64 lim2 = !whole && !graph ? CS_NO_LIMIT : ctx->visc == -1 && std::is_same<T, float>::value ? 4096 : 2400;
+    return coarse_first(ctx, (int)M.s.size(), dim == 2 ? lim2 : CS_NO_LIMIT, [&](int l) { return M.s[l].g.nc; },
                         [&](int l) { return (size_t)(3 * dim) * (size_t)M.s[l].g.nc * sizeof(T); });
 }
 
 template <typename T>
-static int cc_coarse_first(fhd_ctx* ctx, Multigrid<T>& M) {
-    return coarse_first(ctx, (int)M.c.size(), ctx->dim == 2 ? 2400 : 4096, [&](int l) { return M.c[l].g.nc; },
+static int cc_coarse_first(fhd_ctx* ctx, Multigrid<T>& M, bool graph) {
+    const i64 lim2 = ctx->fused_mode == 0 && !graph ? CS_NO_LIMIT : 2400;
+    return coarse_first(ctx, (int)M.c.size(), ctx->dim == 2 ? lim2 : 4096, [&](int l) { return M.c[l].g.nc; },
                         [&](int l) { return (size_t)3 * (size_t)M.c[l].g.nc * sizeof(T); });
 }
 
@@ -948,7 +956,7 @@ static int stag_vcycle(fhd_ctx* ctx, Multigrid<T>& M, bool zero0) {
     const int dim = ctx->dim;
     cudaStream_t st = ctx->stream;
     // levels from lc down run in the coarse kernel, which zeroes their phi
-    const int lc = stag_coarse_first(ctx, M);
+    const int lc = stag_coarse_first(ctx, M, ctx->capturing);
     const int lt = lc < nl - 1 ? lc : nl - 1;  // last level of the per-level descent
     // a level that starts from zero by the z-march does not store the zeros
     const int nd = ctx->p.stag_mg_nsmooths_down;
@@ -1426,7 +1434,7 @@ static int tune_levels_locked(fhd_ctx* ctx, Multigrid<T>& M, std::vector<T*>& sc
         }
         return 0;
     };
-    const int lcs = stag_coarse_first(ctx, M), lcc = cc_coarse_first(ctx, M);
+    const int lcs = stag_coarse_first(ctx, M, true), lcc = cc_coarse_first(ctx, M, true);
     const i64 nc_max = ctx->g0.nc;
     for (int l = 0; l < (int)M.s.size(); l++) {
         StagLevel<T>& L = M.s[l];
@@ -1675,7 +1683,7 @@ static int cc_cycles(fhd_ctx* ctx, Multigrid<T>& M) {
     CCLevel<T>& C = M.c[0];
     const i64 nc = C.g.nc;
     const int maxv = ctx->p.mg_max_vcycles;
-    const int lc = cc_coarse_first(ctx, M);
+    const int lc = cc_coarse_first(ctx, M, ctx->capturing);
     const bool zero = maxv == 1 && cc_from_zero(ctx, M, 0, lc);
     if (!zero) FHD_CUDA_TRY(cudaMemsetAsync(C.phi, 0, sizeof(T) * nc, ctx->stream));
     double r0 = 1.0;
