@@ -158,6 +158,7 @@ static int build_mg(fhd_ctx* ctx, Multigrid<T>& M) {
         }
         L.zm_ok = dim == 2 ? all_even(L.g) && nc < (1ll << 31)
                            : stag_zm_pick<T>(L.g, 1, ctx->sms, L.zm[0]) && stag_zm_pick<T>(L.g, 2, ctx->sms, L.zm[1]);
+        L.zm_work = dim == 3 && L.zm_ok && nc > (1 << 19) ? zm_work(L.g, L.zm[1]) : 0.0;
     }
     const int ncl = nlevs_mg(ctx->g0, ctx->p.mg_minwidth);
     M.c.resize(ncl);
@@ -657,16 +658,23 @@ static int stag_smooths_planned(fhd_ctx* ctx, StagLevel<T>& L, const SmoothPlan&
 // without cross terms (zm_shape, all that the process's plan table may go by);
 // not where a caller forced or imported a plan, or asked for colour launches
 // (fhd_ctx_set_fused 0), or where an array is not aligned.  It is the fastest
-// form at every size it takes (a pair of smooths, FP32, before and now: 40^3
-// 52 -> 9 us, 128^3 64 -> 44, 192^3 238 -> 113, 256^3 349 -> 280; FP64 128^3
-// 136 -> 99), so no plan is timed against it.
+// form of all levels but large thin slabs (a pair of smooths, FP32, before and
+// now: 40^3 52 -> 9 us, 128^3 64 -> 44, 192^3 238 -> 113, 256^3 349 -> 280; FP64
+// 128^3 136 -> 99), so no plan is timed against it.  Slabs of more than 2^19
+// cells whose march works on more than 3.2 pairs for each one it stores are
+// timed against the candidates, and above 4 the fixed rules leave them to the
+// colours (a V-cycle in us, best candidate and march; FP64 1024^2 x 4, 6.6 pairs:
+// 1162, 1715; 512^2 x 6, 4.4: 836, 938; 512^2 x 10, 3.4: 1095, 1166; 512^2 x 12,
+// 3.1: 1252, 1235; FP32 2048 x 1024 x 4, 5.8: 1669, 1982; 1024^2 x 6, 3.8: 1742,
+// 1807; 1024^2 x 8, 3.2: 1754, 1615).
 template <typename T>
 static bool zm_shape(fhd_ctx* ctx, const StagLevel<T>& L) {
     return L.zm_ok && ctx->visc == 1 && ctx->p.stag_mg_smoother != 0 && !ctx->has_walls;
 }
 template <typename T>
 static bool zm_use(fhd_ctx* ctx, const StagLevel<T>& L) {
-    return zm_shape(ctx, L) && ctx->fused_mode != 0 && (L.plan.kind < 0 || L.plan.march) && stag_aligned(L, ctx->dim);
+    return zm_shape(ctx, L) && ctx->fused_mode != 0 && (L.plan.kind < 0 ? L.zm_work <= 4.0 : L.plan.march) &&
+           stag_aligned(L, ctx->dim);
 }
 
 // one launch of ns smooths phi -> tmp of every component; the two buffers
@@ -1480,23 +1488,30 @@ static int tune_levels_locked(fhd_ctx* ctx, Multigrid<T>& M, std::vector<T*>& sc
             S.rhs[c] = scratch[2 * dim + c];
         }
         if (!stag_aligned(S, dim)) continue;
-        if (can_march) {  // fastest wherever it runs (zm_use): timed for the record only
+        if (can_march) {
             S.plan = march;
             if (int rc = time_pairs(ctx, ev[0], ev[1], [&]() { return stag_zm_launch(ctx, S, 2, 0); }, march.us))
                 return rc;
-            L.plan = march;
-            g_tune[key] = L.plan;
-            continue;
+            if (L.zm_work <= 3.2) {  // the fastest (zm_use): timed for the record only
+                L.plan = march;
+                g_tune[key] = L.plan;
+                continue;
+            }
         }
         int best = -1;
         for (size_t i = 0; i < cands.size(); i++) {
             float us = 0.f;
-            if (cands[i].kind == 2) continue;  // (a level it takes marches)
+            if (cands[i].kind == 2) continue;  // (behind the march where that is the fastest, and no slab's plan)
             if (int rc = time_pairs(ctx, ev[0], ev[1], [&]() { return stag_smooths_planned(ctx, S, cands[i], 2); },
                                     us))
                 return rc;
             cands[i].us = us;
             if (best < 0 || us < cands[best].us) best = (int)i;
+        }
+        if (can_march && march.us <= cands[best].us) {
+            L.plan = march;
+            g_tune[key] = L.plan;
+            continue;
         }
         L.plan = cands[best];
         L.plan.ncand = (int)cands.size();

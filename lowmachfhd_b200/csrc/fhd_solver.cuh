@@ -181,6 +181,7 @@ struct StagLevel {
     // the level's shape takes it
     bool zm_ok = false;
     ZMGeom zm[2];
+    double zm_work = 0.0;  // large 3D levels: pairs worked on for each one stored (zm_work)
     bool away = false;  // phi and tmp are exchanged
     // the visc_type 1 diagonal alpha_scale alpha + 2 dim beta q, staged by the
     // row-tile smoother in place of alpha (allocated when a plan takes it)

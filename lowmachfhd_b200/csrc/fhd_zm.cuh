@@ -291,6 +291,12 @@ inline bool zm_geom(const Grid& g, int ns, int ip, int TY, int KZ, int maxt, int
     return true;
 }
 
+// pairs that the blocks of a march work on, rings and run-in included, for each
+// pair that they store
+inline double zm_work(const Grid& g, const ZMGeom& G) {
+    return (double)G.threads * G.tx * G.ty * G.chunks * (G.KZ + 4 * G.ns) / ((double)G.np * g.n[1] * g.n[2]);
+}
+
 // The tile and the z-runs of a level: the least of waves x plane steps x
 // cycles per step.  One block runs on an SM at a time (its shared memory);
 // a step takes as long as its warps need to issue (per_warp cycles each), or
