@@ -157,7 +157,8 @@ static int build_mg(fhd_ctx* ctx, Multigrid<T>& M) {
             }
         }
         L.zm_ok = dim == 2 ? all_even(L.g) && nc < (1ll << 31)
-                           : stag_zm_pick<T>(L.g, 1, ctx->sms, L.zm[0]) && stag_zm_pick<T>(L.g, 2, ctx->sms, L.zm[1]);
+                           : ctx->visc == 1 && stag_zm_pick<T>(L.g, 1, ctx->sms, L.zm[0]) &&
+                                 stag_zm_pick<T>(L.g, 2, ctx->sms, L.zm[1]);
         L.zm_work = dim == 3 && L.zm_ok && nc > (1 << 19) ? zm_work(L.g, L.zm[1]) : 0.0;
     }
     const int ncl = nlevs_mg(ctx->g0, ctx->p.mg_minwidth);

@@ -315,8 +315,10 @@ inline bool zm_pick(const Grid& g, int ns, int sms, int ncomp, int maxt, int per
             ZMGeom G;
             if (!zm_geom(g, ns, ip, TY, g.n[2] & ~1, maxt, per_thread, G)) continue;
             const double step = per_warp * (G.threads / 32) > least ? per_warp * (G.threads / 32) : least;
-            // as many z-runs as fill one, two, .. waves
+            // as many z-runs as fill one, two, .. waves; no split of a tile takes
+            // less than its planes spread over the SMs
             const long tiles = (long)G.tx * G.ty * ncomp;
+            if (cost >= 0.0 && (double)tiles * g.n[2] / sms * step >= cost) continue;
             int last = 0;
             for (long w = 1; w <= tiles / sms + 4; w++) {
                 const long ch = w * sms / tiles;
