@@ -735,8 +735,8 @@ __device__ __forceinline__ void stag_coarse_run(const StagCoarseArgs<T>& a) {
     }
 }
 
-template <typename T, int DIM, int VISC, bool WALL = false>
-__global__ void __launch_bounds__(CS_THREADS) k_stag_coarse(const __grid_constant__ StagCoarseArgs<T> a) {
+template <typename T, int DIM, int VISC, bool WALL = false, int NT = CS_THREADS>
+__global__ void __launch_bounds__(NT) k_stag_coarse(const __grid_constant__ StagCoarseArgs<T> a) {
     stag_coarse_run<T, DIM, VISC, WALL>(a);
 }
 

@@ -950,6 +950,21 @@ static int stag_coarse(fhd_ctx* ctx, Multigrid<T>& M, int lc) {
     }
     with_dim_visc(dim, ctx->visc, [&](auto D, auto V) {
         constexpr int DIM = decltype(D)::value, VISC = decltype(V)::value;
+        // a large odd bottom of the other viscosity types, swept in two passes
+        // per colour, feeds 1024 threads (2D, us per stag_mg_solver call with 512
+        // and 1024: visc_type 2 FP64 35 x 49 141, 128, 45 x 63 186, 167, 47^2 174,
+        // 153; 3 FP32 51 x 90 285, 253); even levels are as fast or faster with 512
+        // (48 x 64 FP64 2: 212, 218), and so are 3D ones
+        if constexpr (DIM == 2 && VISC != 1) {
+            const Grid& gb = a.g[a.nlev - 1];
+            if (!all_even(gb) && gb.nc > 1024) {
+                rc |= rb_allow_smem(k_stag_coarse<T, DIM, VISC, false, 1024>, smem);
+                if (rc) return;
+                k_stag_coarse<T, DIM, VISC, false, 1024><<<1, 1024, smem, ctx->stream>>>(a);
+                rc |= post(ctx);
+                return;
+            }
+        }
         rc |= rb_allow_smem(k_stag_coarse<T, DIM, VISC>, smem);
         if (rc) return;
         k_stag_coarse<T, DIM, VISC><<<1, CS_THREADS, smem, ctx->stream>>>(a);
