@@ -1333,7 +1333,7 @@ static int cc_smooths(fhd_ctx* ctx, CCLevel<T>& C, int count, int zero = 0, bool
 // shapes, the tiled fused smooth with several tile sizes, the row-tile
 // smooth with every tile height that fits -- are timed once per process,
 // device and level shape with CUDA events, and the fastest is kept.  The
-// timing runs on scratch unknowns and right-hand sides (zero) with the
+// timing runs on scratch unknowns (zero at first) and right-hand sides (one) with the
 // level's own prepared coefficients, before any capture, so a solve's data
 // is never touched.  Every plan evaluates the same update expression on the
 // same operands in the same colour order: the choice changes time only.
@@ -1446,15 +1446,22 @@ template <typename T>
 static int tune_levels_locked(fhd_ctx* ctx, Multigrid<T>& M, std::vector<T*>& scratch, cudaEvent_t ev[2]) {
     const int dim = ctx->dim;
     const int force = ctx->tune_mode >= 2 ? ctx->tune_mode - 2 : -1;
-    // scratch unknowns, right-hand sides and second buffers: 3 dim arrays of
-    // the largest level timed, zeroed
+    // scratch unknowns, second buffers and right-hand sides: 3 dim arrays of
+    // the largest level timed, zero but for right-hand sides of one (an FP64
+    // quotient of zero takes longer than a solve's: 256^3, a pair of smooths by
+    // the march, 1217 us on zeros, 658 in a solve)
     auto get_scratch = [&](i64 nc) -> int {
         if (!scratch.empty()) return 0;
         for (int i = 0; i < 3 * dim; i++) {
             void* p = nullptr;
             FHD_CUDA_TRY(cudaMallocAsync(&p, (size_t)nc * sizeof(T), ctx->stream));
             scratch.push_back((T*)p);
-            FHD_CUDA_TRY(cudaMemsetAsync(p, 0, (size_t)nc * sizeof(T), ctx->stream));
+            if (i < 2 * dim) {
+                FHD_CUDA_TRY(cudaMemsetAsync(p, 0, (size_t)nc * sizeof(T), ctx->stream));
+            } else {
+                k_fill<T><<<flat_blocks(nc), 256, 0, ctx->stream>>>(nc, (T*)p, T(1));
+                FHD_POST(ctx);
+            }
         }
         return 0;
     };
@@ -1576,7 +1583,7 @@ static int tune_levels_locked(fhd_ctx* ctx, Multigrid<T>& M, std::vector<T*>& sc
         CCLevel<T> S = C;
         S.phi = scratch[0];
         S.tmp = scratch[1];
-        S.rhs = scratch[2];
+        S.rhs = scratch[2 * dim];
         if (can_march) {  // fastest wherever it runs (cc_t2_use): timed for the record only
             S.plan = march;
             if (int rc = time_pairs(ctx, ev[0], ev[1], [&]() { return cc_t2_launch(ctx, S, 2, 0); }, march.us))
