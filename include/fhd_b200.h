@@ -199,8 +199,8 @@ int fhd_ctx_set_graphs(fhd_ctx* ctx, int mode);
  * whose unknowns, right-hand sides and residuals fit in one SM's shared
  * memory down to the bottom, up to the sizes where launches are faster) as one
  * single-block kernel per V-cycle instead of one launch per smoother colour
- * and transfer (mode 1 or -1 default: on, 0: per-level launches).  Same arithmetic either way.  Replaces no
- * reference routine: the levels are those of stag_mg_solver.f90:301-599 and
+ * and transfer (mode 1 or -1 default: on, 0: per-level launches).  Same
+ * arithmetic either way.  Replaces no reference routine: the levels are those of stag_mg_solver.f90:301-599 and
  * of the pressure multigrid behind macproject.f90:294-298. */
 int fhd_ctx_set_coarse(fhd_ctx* ctx, int mode);
 /* Whole smooths (both colours of every component, one or two smooths per
@@ -229,16 +229,17 @@ int fhd_ctx_set_fused(fhd_ctx* ctx, int mode);
 int fhd_ctx_set_wall_speed(fhd_ctx* ctx, const double wallspeed_lo[6], const double wallspeed_hi[6]);
 /* Smoother autotuner.  Each multigrid level that smooths through launches
  * (staggered and pressure multigrids, above the single-block coarse end) can
- * smooth as colour launches with one of four thread-block shapes, as the
- * tiled fused smooth with one of several tile sizes (3D), or as the row-tile
- * smooth with one of the tile heights that fit, one CTA per SM with a deep
- * copy ring (256 or 512 compute threads) or two with a short one (3D FP32
- * visc_type 1).  Levels that fhd_ctx_set_fused's march or tiles take use
- * those, one past the candidate list, timed for the record only.  With
- * the tuner on (mode 1 or -1 default), the first solve call that meets a
- * level shape times every candidate on scratch unknowns with the level's
- * coefficients and keeps the fastest for the process (per device,
- * precision, visc_type and shape); later calls and contexts reuse it.
+ * smooth as colour launches with one of four thread-block shapes or as the
+ * tiled fused smooth with one of several tile sizes (3D).  With the tuner on
+ * (mode 1 or -1 default), the first solve call that meets a level shape times
+ * these candidates on scratch unknowns with the level's coefficients and keeps
+ * the fastest for the process (per device, precision, visc_type and shape);
+ * later calls and contexts reuse it.  Levels that fhd_ctx_set_fused's march or
+ * tiles take use those, one past the candidate list, timed for the record only;
+ * large thin slabs time the march against the candidates.  The row-tile smooth
+ * (3D FP32 visc_type 1: one of the tile heights that fit, one CTA per SM with a
+ * deep copy ring and 256 or 512 compute threads, or two with a short one) is in
+ * the list for forced and imported plans and never chosen by time.
  * Mode 0: the fixed size rules of fhd_ctx_set_fused.  Mode 2 + k: candidate
  * k of every level (its first where it has fewer), untimed, for tests.
  * Every candidate evaluates the update expression of the colour sweeps of
@@ -251,8 +252,8 @@ int fhd_ctx_set_tune(fhd_ctx* ctx, int mode);
  * shape of their two smooths per launch), 2 row-tile; ncand candidates
  * considered; pair_us the measured time of one smooth pair (0 when not
  * timed); shape = {block x, block y, 0, 1, threads} for colour launches,
- * {tile x, tile y, z-runs, CTAs per SM, compute threads} for fused smooths.  Any output pointer may be NULL.  No
- * reference counterpart. */
+ * {tile x, tile y, z-runs, CTAs per SM, compute threads} for fused smooths.
+ * Any output pointer may be NULL.  No reference counterpart. */
 int fhd_ctx_tune_info(fhd_ctx* ctx, int which, int level, int* kind, int* ncand, double* pair_us,
                       int shape[5]);
 /* The candidate list the tuner would time for one level (host only, no

@@ -6,11 +6,10 @@
 // stag_mg_solver V-cycle (stag_mg_solver.f90:301-599) and of the pressure
 // V-cycle behind macproject (macproject.f90:294-298) is a dependent launch
 // that moves a few kilobytes.  These kernels run every level from the first
-// one whose arrays fit in shared memory down to the bottom inside one CTA
-// of 512 threads: the unknowns, right-hand sides and residuals of all
-// those levels live in shared memory, the read-only coefficients come
-// through the L1 (non-coherent loads), and a __syncthreads() replaces each
-// launch boundary.
+// one whose arrays fit in shared memory (up to the cell limits of the host's
+// coarse_first) down to the bottom inside one CTA of 512 threads: the unknowns,
+// right-hand sides and residuals of all those levels live in shared memory, and
+// a __syncthreads() replaces each launch boundary.
 //
 // Arithmetic is the same as the per-level kernels: the operator, smoother
 // update, restriction and prolongation are the shared expressions of
@@ -29,15 +28,17 @@
 //     steps per smooth instead of four (2D) or six (3D);
 //   * only as many warps as a level has pairs take part in its sweeps, down
 //     to one warp and no block barrier;
-//   * coefficients come from shared memory: the staggered diagonal lies in
-//     the scratch array between two residuals, the pressure coefficients
-//     beside the unknowns on every level that has room;
+//   * coefficients come from shared memory: the staggered diagonal of
+//     visc_type 1 lies in the scratch array between two residuals, the pressure
+//     coefficients beside the unknowns on every level that has room (a large
+//     bottom may have none); the other viscosity types read theirs through the
+//     L1 by non-coherent loads;
 //   * transfers run one thread per coarse cell, whose coarse values and
 //     indices serve all its children;
 //   * an odd level (the colours meet across the wrap) is swept from one
 //     buffer into the other, one step per colour.
 // The other viscosity types and the Jacobi smoother keep components apart
-// and cells in index order.
+// and cells in index order; an odd level takes them two passes per colour.
 //
 // One call before (1024 threads, a step per component and colour) and now:
 // staggered FP32 16^3 down 133 -> 52 us, 10^3 down 81 -> 21, FP64 32^2 down

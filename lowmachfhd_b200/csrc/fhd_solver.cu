@@ -846,8 +846,9 @@ static int stag_residual(fhd_ctx* ctx, StagLevel<T>& L) {
     return rc;
 }
 
-// shared memory one coarse kernel may take: the device's opt-in limit less a
-// margin for the L1 that caches the coefficients
+// shared memory the unknowns, right-hand sides and scratch of one coarse kernel
+// may take.  The pressure kernel's coefficients then fill what is left up to
+// the device's opt-in limit (cc_coarse_layout).
 static size_t coarse_smem_cap() {
     int dev = 0, optin = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
@@ -1330,9 +1331,12 @@ static int cc_smooths(fhd_ctx* ctx, CCLevel<T>& C, int count, int zero = 0, bool
 // ---------------------------------------------------------------------
 // For every level that smooths through launches (above the single-CTA
 // coarse end), the candidate plans -- colour launches with four thread-block
-// shapes, the tiled fused smooth with several tile sizes, the row-tile
-// smooth with every tile height that fits -- are timed once per process,
-// device and level shape with CUDA events, and the fastest is kept.  The
+// shapes, the tiled fused smooth with several tile sizes -- are timed once per
+// process, device and level shape with CUDA events, and the fastest is kept.
+// Levels that the z-march or the 2D tiles take use those without a contest
+// (timed for the record), large thin slabs after one (zm_use).  The row-tile
+// smooth stands in the candidate lists too, for forced and imported plans only:
+// the march is faster on every level that it could take.  The
 // timing runs on scratch unknowns (zero at first) and right-hand sides (one) with the
 // level's own prepared coefficients, before any capture, so a solve's data
 // is never touched.  Every plan evaluates the same update expression on the

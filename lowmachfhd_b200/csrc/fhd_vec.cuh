@@ -73,8 +73,8 @@ __device__ __forceinline__ void red_finish(double v, RedSlot rs) {
 
 // ---------------------------------------------------------------------
 // Orthogonalisation of a new Krylov vector w against i others
-// (gmres.f90:352-389), two passes over the vectors instead of one per
-// vector.  Modified Gram-Schmidt takes h_k = <w - sum_{j<k} h_j v_j, v_k>,
+// (gmres.f90:352-389), two passes over the vectors, GS_MAXV at a time, instead of
+// one per vector.  Modified Gram-Schmidt takes h_k = <w - sum_{j<k} h_j v_j, v_k>,
 // that is h_k = <w, v_k> - sum_{j<k} h_j <v_j, v_k>: all products <w, v_k> and
 // the new row of <v_j, v_k> come from one pass (k_gs_dots, whose last block
 // solves for h), and w - sum h_k v_k with its norm from a second
@@ -83,8 +83,10 @@ __device__ __forceinline__ void red_finish(double v, RedSlot rs) {
 //
 // The vectors are kept as computed (u_k, with n2_k = |u_k|^2) rather than
 // scaled to length one: v_k = u_k / |u_k| enters through its coefficients,
-// and the operator scales its result (k_stokes_apply's inv).  So a step moves
-// 2 i + 3 vectors where one pass per vector and the scaling moved 4 i + 3.
+// and the operator scales its result (k_stokes_apply's inv).  So a step of
+// i <= GS_MAXV moves 2 i + 3 vectors where one pass per vector and the scaling
+// moved 4 i + 3; every further GS_MAXV vectors read w, u_{i-1} and the partly
+// updated vector again and write it, 4 more.
 //
 // Bound: DRAM (192^3, five vectors: dots 279 us, update 281 us for 1.6 GB,
 // 5.6 TB/s).  Seven steps of the 192^3 solve with their norms: 5.2 ms one

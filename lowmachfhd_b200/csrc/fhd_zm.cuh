@@ -18,9 +18,12 @@
 // wrap inside the tile and need no ring in x.
 //
 // Bounds.  Two smooths per launch move the unknown, the right-hand side and
-// alpha once instead of twice (256^3: 838 MB of DRAM traffic for two smooths);
-// what limits it now is issue: about 144 instructions per pair and plane step,
-// a third of them the stencil's arithmetic, at 2.2 per cycle.  Staging by
+// alpha once instead of twice (256^3: 883 MB of DRAM traffic for two smooths);
+// what limits it now is the chain of a step's four stages, which 20 to 28 warps
+// an SM (15 in FP64) do not hide: 132 instructions per pair and plane step (FP64
+// 172), a third of them the stencil's arithmetic, on 58 % of the issue slots (43
+// %), DRAM at 33 % (28 %); of the 8.7 cycles between two issues of a warp 2.6 wait
+// for shared memory and 1.6 for the pipeline (1.5 and 2.8).  Staging by
 // asynchronous copies three planes ahead, each thread its own pair, took the
 // 256^3 pair from 338 to 280 us over register prefetch; unrolling by four
 // planes, so that no value is moved between registers, and dropping the
@@ -298,8 +301,10 @@ inline double zm_work(const Grid& g, const ZMGeom& G) {
 }
 
 // The tile and the z-runs of a level: the least of waves x plane steps x
-// cycles per step.  One block runs on an SM at a time (its shared memory);
-// a step takes as long as its warps need to issue (per_warp cycles each), or
+// cycles per step.  One block is counted per SM at a time: FP64 blocks of two
+// smooths fill its shared memory (128 KB), FP32 ones (112 KB) of more than 448
+// threads its registers; smaller FP32 tiles may pair, which the model leaves out.
+// A step takes as long as its warps need to issue (per_warp cycles each), or
 // the chain of a step's stages when they are few (least).
 inline bool zm_pick(const Grid& g, int ns, int sms, int ncomp, int maxt, int per_thread, double per_warp,
                     double least, ZMGeom& best) {
